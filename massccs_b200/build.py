@@ -47,7 +47,11 @@ def _run(cmd):
     return r
 
 
-ENGINE_UNITS = ["ccs_engine.cu", "field.cu", "traj_field.cu", "setup_gpu.cu"]
+# (source, defines, object): the trajectory passes are compiled once per precision and gas shape
+ENGINE_UNITS = [("ccs_engine.cu", [], "ccs_engine.o"), ("field.cu", [], "field.o"),
+                ("traj_field.cu", [], "traj_field.o"), ("setup_gpu.cu", [], "setup_gpu.o")]
+ENGINE_UNITS += [(f"{src}.cu", [f"-DCCS_PASS_T={t}", f"-DCCS_PASS_GAS={g}"], f"{src}_{t}_{g}.o")
+                 for src in ("lane_pass", "warp_pass") for t in ("float", "double") for g in (0, 1, 2)]
 ENGINE_HEADERS = ["ccs_device.cuh", "field_device.cuh", "engine_ctx.h"]
 
 
@@ -60,16 +64,16 @@ def build_engine(force=False, verbose=False):
     out = os.path.join(LIB, "libmassccs_gpu.so")
     headers = [os.path.join(CSRC, f) for f in ENGINE_HEADERS] + [os.path.join(INC, "massccs_gpu.h")]
     objs, todo = [], []
-    for u in ENGINE_UNITS:
+    for u, defines, name in ENGINE_UNITS:
         src = os.path.join(CSRC, u)
-        obj = os.path.join(obj_dir, u.replace(".cu", ".o"))
+        obj = os.path.join(obj_dir, name)
         objs.append(obj)
         if force or _newer(obj, [src] + headers):
-            cmd = [_nvcc()] + ARCH + NVCC_FLAGS + ["-c", "-o", obj, src]
+            cmd = [_nvcc()] + ARCH + NVCC_FLAGS + defines + ["-c", "-o", obj, src]
             if verbose:
                 cmd += ["-Xptxas", "-v"]
             todo.append(cmd)
-    with ThreadPoolExecutor(max_workers=max(1, len(todo))) as ex:
+    with ThreadPoolExecutor(max_workers=max(1, min(len(todo), os.cpu_count() or 1))) as ex:
         for r in ex.map(_run, todo):
             if verbose:
                 sys.stderr.write(r.stderr)

@@ -37,6 +37,22 @@ constexpr double BOLTZMANN_K = 1.38064E-23;
 constexpr double OMEGA_TO_FS_INV = 2.45400505E8;
 constexpr double PI_D = 3.14159265358979323846;
 
+// The launch parameters that the kernels compute with, in the precision they
+// compute in.  KParams holds them as doubles; a conversion at each use cost
+// the step an F2F (a quarter-rate instruction) per constant, so the host
+// converts them once (the same rounding, so the same results).
+template <typename T> struct KConst {
+  T ox, oy, oz, h, inv_h;
+  T bb_lo[3], bb_hi[3], reach;
+  T kq[3];  // KCOUL * charge of each gas site
+  T rlj2, rc2, rc6inv, rc12inv, rc3inv, c1, c2, alpha;
+  T ref_corner[3], ref_inv_h;
+  T ref_lim[3];  // a point within this of the origin on every axis is inside the reference grid
+  T d2, mu, lx, ly, lz, inv_a, inv_b, inv_c;
+  T gas_m[3], m2M, m0M;
+  T half_kconv_over_m1, half_kconv_over_m2, inv_m1, inv_m2, mu12, mu12_over_m1, mu12_over_m2;
+};
+
 // Per-launch parameters (passed by value).
 struct KParams {
   // target atoms, sorted by engine cell (z fastest within a column)
@@ -112,7 +128,43 @@ struct KParams {
   unsigned long long spec_max_parked;  // speculate only when at most this many were parked
   int *error;                 // 1 = watchdog, 2 = a tensor-core stage timed out
   FieldK field;               // learned field (field.on == 0: every force exact)
+  int lane_width;             // lane pass: trajectories per warp (1..32)
+  KConst<float> k32;
+  KConst<double> k64;
 };
+
+template <typename T> __host__ __device__ __forceinline__ const KConst<T> &kconst(const KParams &kp) {
+  if constexpr (sizeof(T) == 4) return kp.k32; else return kp.k64;
+}
+template <typename T> __host__ __device__ __forceinline__ KConst<T> &kconst(KParams &kp) {
+  if constexpr (sizeof(T) == 4) return kp.k32; else return kp.k64;
+}
+
+// Fills the typed constants from the double ones.
+template <typename T> inline void fill_kconst(KParams &kp) {
+  KConst<T> &k = kconst<T>(kp);
+  k.ox = T(kp.ox); k.oy = T(kp.oy); k.oz = T(kp.oz); k.h = T(kp.h); k.inv_h = T(kp.inv_h);
+  k.reach = T(kp.reach);
+  k.rlj2 = T(kp.rlj2); k.rc2 = T(kp.rc2); k.rc6inv = T(kp.rc6inv); k.rc12inv = T(kp.rc12inv);
+  k.rc3inv = T(kp.rc3inv); k.c1 = T(kp.c1); k.c2 = T(kp.c2); k.alpha = T(kp.alpha);
+  k.ref_inv_h = T(kp.ref_inv_h);
+  const int n[3] = {kp.ref_nx, kp.ref_ny, kp.ref_nz};
+  for (int d = 0; d < 3; d++) {
+    k.bb_lo[d] = T(kp.bb_lo[d]); k.bb_hi[d] = T(kp.bb_hi[d]);
+    k.kq[d] = T(KCOUL * kp.q_site[d]);
+    k.ref_corner[d] = T(kp.ref_corner[d]);
+    // half the grid's edge less 0.01 A: far more than the rounding of the index
+    k.ref_lim[d] = T(0.5 * n[d] * kp.ref_h - 0.01);
+    k.gas_m[d] = T(kp.gas_m[d]);
+  }
+  k.m2M = k.gas_m[1] / T(kp.gas_mass); k.m0M = k.gas_m[0] / T(kp.gas_mass);
+  k.d2 = T(kp.d_bond * kp.d_bond); k.mu = T(kp.mu);
+  k.lx = T(kp.lx); k.ly = T(kp.ly); k.lz = T(kp.lz);
+  k.inv_a = T(kp.inv_a); k.inv_b = T(kp.inv_b); k.inv_c = T(kp.inv_c);
+  k.half_kconv_over_m1 = T(kp.half_kconv_over_m1); k.half_kconv_over_m2 = T(kp.half_kconv_over_m2);
+  k.inv_m1 = T(kp.inv_m1); k.inv_m2 = T(kp.inv_m2); k.mu12 = T(kp.mu12);
+  k.mu12_over_m1 = T(kp.mu12_over_m1); k.mu12_over_m2 = T(kp.mu12_over_m2);
+}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -162,13 +214,21 @@ constexpr int SPEC_FROM_MIN = 2;  // the fewest failed tries after which specula
 constexpr int SPEC_SLOTS = 9 - SPEC_FROM_MIN;  // tries tries..tries+6 (those above 8 are skipped)
 
 template <typename T> struct Real;
+// fma/mul/add: single roundings that the compiler neither fuses nor splits,
+// where one expression must round alike in every kernel that has it.
 template <> struct Real<float> {
+  static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+  static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
   static __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
   static __device__ __forceinline__ float sq(float x) { return sqrtf(x); }
   // quotient for the FP32 integrator (2 ulp; the operands are O(1) and positive-definite)
   static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
 };
 template <> struct Real<double> {
+  static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+  static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+  static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
   static __device__ __forceinline__ double sq(double x) { return sqrt(x); }
   static __device__ __forceinline__ double div(double a, double b) { return a / b; }
@@ -197,6 +257,12 @@ template <int GAS> struct GasShape;
 template <> struct GasShape<GAS_ATOM> { static constexpr int NS = 1, DIP = 0; };
 template <> struct GasShape<GAS_N2> { static constexpr int NS = 3, DIP = 2; };
 template <> struct GasShape<GAS_CO2> { static constexpr int NS = 3, DIP = 1; };
+
+template <int GAS> struct Sites {
+  static constexpr int NS = GasShape<GAS>::NS;
+  static constexpr int pa = 0, pb = GAS == GAS_CO2 ? 2 : 1, pc = GAS == GAS_CO2 ? 1 : 2;
+  static constexpr int cs = GAS == GAS_ATOM ? 0 : pc;  // reference point of the reach sphere
+};
 
 // Site layout: which sites carry LJ, and with which parameter set.
 template <int GAS> __device__ __forceinline__ constexpr int site_lj(int s) {
@@ -252,12 +318,21 @@ template <int G, typename T> __device__ __forceinline__ T group_sum(T v, unsigne
 // weighted by the switch S(r) (field_device.cuh), its force by
 // -grad(S u) = S F - u S'(r) d / r, the dipole's field by S e and its
 // Jacobian by grad(S e) (still symmetric, since e is along d).
-template <typename T, int GAS, bool HASQ, bool SPLIT = false>
+//
+// WF, WU: which sums are wanted.  The energies are used only when a try
+// begins or ends (its energy test), so the steps between leave them out: a
+// quarter of the arithmetic, the compensated additions' serial chain with it.
+//
+// DIPF: how the Coulomb term of the dipole's site rounds 1/r^3 - 1/rc^3 (the
+// captured orbits amplify one rounding to another outcome, so each pass keeps
+// one form for good): fused (true) or with 1/r^3 rounded first.
+template <typename T, int GAS, bool HASQ, bool SPLIT = false, bool WF = true, bool WU = true, bool DIPF = false>
 __device__ __forceinline__ void visit_atom(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
                                            const bool (&act)[GasShape<GAS>::NS], const Atom<T> &a,
                                            Acc<T, GasShape<GAS>::NS> &acc) {
   constexpr int NS = GasShape<GAS>::NS;
-  const T rlj2 = T(kp.rlj2), rc2 = T(kp.rc2);
+  const KConst<T> &kc = kconst<T>(kp);
+  const T rlj2 = kc.rlj2, rc2 = kc.rc2;
 #pragma unroll
   for (int s = 0; s < NS; s++) {
     if (!act[s]) continue;
@@ -278,35 +353,41 @@ __device__ __forceinline__ void visit_atom(const KParams &kp, const T (&p)[GasSh
       const bool in_lj = r2 < rlj2;
       const T A = lj == 2 ? a.Ac : a.A, B = lj == 2 ? a.Bc : a.B;
       const T ir6 = ir2 * ir2 * ir2;
-      const T u = in_lj ? ir6 * (A * ir6 - B) - (A * T(kp.rc12inv) - B * T(kp.rc6inv)) : T(0);
-      T fl = in_lj ? ir6 * (T(12) * A * ir6 - T(6) * B) * ir2 : T(0);
+      T u = T(0);
+      if constexpr (WU || SPLIT) u = in_lj ? ir6 * (A * ir6 - B) - (A * kc.rc12inv - B * kc.rc6inv) : T(0);
+      T fl = T(0);
+      if constexpr (WF) fl = in_lj ? ir6 * (T(12) * A * ir6 - T(6) * B) * ir2 : T(0);
       if constexpr (SPLIT) {
         fl = sw * fl - u * dsw;
         us += sw * u;
-      } else {
+      } else if constexpr (WU) {
         us += u;
       }
-      acc.f[s][0] += fl * dx; acc.f[s][1] += fl * dy; acc.f[s][2] += fl * dz;
+      if constexpr (WF) { acc.f[s][0] += fl * dx; acc.f[s][1] += fl * dy; acc.f[s][2] += fl * dz; }
     }
     if constexpr (HASQ) {
       const bool in_c = r2 < rc2;
-      const T ir3 = ir * ir2;
+      const T ir3 = Real<T>::mul(ir, ir2);
+      const T ir3s = Real<T>::add(ir3, -kc.rc3inv);  // 1/r^3 - 1/rc^3
       if (site_coul<GAS>(s) && kp.coul_on) {
         // Force.cpp:671-683: U = k qi qj (1/r - 3/(2rc) + r^2/(2rc^3)), F = k qi qj (1/r^3 - 1/rc^3) d
-        const T kq = T(KCOUL * kp.q_site[s]) * a.q;
-        const T u = in_c ? kq * (ir - T(kp.c1) + T(kp.c2) * r2) : T(0);
-        T fc = in_c ? kq * (ir3 - T(kp.rc3inv)) : T(0);
+        const T ir3c = DIPF || s != GasShape<GAS>::DIP ? Real<T>::fma(ir, ir2, -kc.rc3inv) : ir3s;
+        const T kq = kc.kq[s] * a.q;
+        T u = T(0);
+        if constexpr (WU || SPLIT) u = in_c ? kq * (ir - kc.c1 + kc.c2 * r2) : T(0);
+        T fc = T(0);
+        if constexpr (WF) fc = in_c ? kq * ir3c : T(0);
         if constexpr (SPLIT) {
           fc = sw * fc - u * dsw;
           us += sw * u;
-        } else {
+        } else if constexpr (WU) {
           us += u;
         }
-        acc.f[s][0] += fc * dx; acc.f[s][1] += fc * dy; acc.f[s][2] += fc * dz;
+        if constexpr (WF) { acc.f[s][0] += fc * dx; acc.f[s][1] += fc * dy; acc.f[s][2] += fc * dz; }
       }
-      if (s == GasShape<GAS>::DIP && kp.dip_on) {
+      if (WF && s == GasShape<GAS>::DIP && kp.dip_on) {
         // Force.cpp:393-426: E += q (1/r^3 - 1/rc^3) d ; dE_ab += q (1/r^3 - 1/rc^3) delta_ab - 3 q d_a d_b / r^5
-        T sq = in_c ? a.q * (ir3 - T(kp.rc3inv)) : T(0);
+        T sq = in_c ? a.q * ir3s : T(0);
         T tq = in_c ? T(-3) * a.q * ir3 * ir2 : T(0);
         if constexpr (SPLIT) {  // E = S e, grad E = S grad e + (S'/r) e d^T
           tq = sw * tq + sq * dsw;
@@ -322,7 +403,7 @@ __device__ __forceinline__ void visit_atom(const KParams &kp, const T (&p)[GasSh
         acc.G[5] += ty * dz;
       }
     }
-    acc.addU(s, us);
+    if constexpr (WU) acc.addU(s, us);
   }
 }
 
@@ -330,10 +411,11 @@ __device__ __forceinline__ void visit_atom(const KParams &kp, const T (&p)[GasSh
 template <typename T>
 __device__ __forceinline__ bool ref_inside(const KParams &kp, T x, T y, T z) {
   if (!kp.ref_check) return true;
-  const T ih = T(kp.ref_inv_h);
-  const int i = (int)floor((x - T(kp.ref_corner[0])) * ih);
-  const int j = (int)floor((y - T(kp.ref_corner[1])) * ih);
-  const int k = (int)floor((z - T(kp.ref_corner[2])) * ih);
+  const KConst<T> &kc = kconst<T>(kp);
+  const T ih = kc.ref_inv_h;
+  const int i = (int)floor((x - kc.ref_corner[0]) * ih);
+  const int j = (int)floor((y - kc.ref_corner[1]) * ih);
+  const int k = (int)floor((z - kc.ref_corner[2]) * ih);
   const long long idx = k + (long long)kp.ref_nz * j + (long long)kp.ref_nz * kp.ref_ny * i;
   return idx >= 0 && idx < (long long)kp.ref_nx * kp.ref_ny * kp.ref_nz;
 }
@@ -346,7 +428,8 @@ __device__ __forceinline__ void column_run(const KParams &kp, int cidx, int ncol
   b = 0;
   len = 0;
   if (cidx >= ncol) return;
-  const T ih = T(kp.inv_h), h = T(kp.h), ox = T(kp.ox), oy = T(kp.oy), oz = T(kp.oz);
+  const KConst<T> &kc = kconst<T>(kp);
+  const T ih = kc.inv_h, h = kc.h, ox = kc.ox, oy = kc.oy, oz = kc.oz;
   const int di = (int)(((float)cidx + 0.5f) * inv_nj);  // exact: cidx < 2^20
   const int i = i0 + di, j = j0 + (cidx - di * nj);
   const T xlo = ox + T(i) * h, ylo = oy + T(j) * h;
@@ -367,7 +450,8 @@ __device__ __forceinline__ void column_run(const KParams &kp, int cidx, int ncol
 template <typename T>
 __device__ __forceinline__ int column_range(const KParams &kp, T cx, T cy, T Rr, int &i0, int &j0, int &nj,
                                             float &inv_nj) {
-  const T ih = T(kp.inv_h), ox = T(kp.ox), oy = T(kp.oy);
+  const KConst<T> &kc = kconst<T>(kp);
+  const T ih = kc.inv_h, ox = kc.ox, oy = kc.oy;
   i0 = (int)fmax(T(0), floor((cx - Rr - ox) * ih));
   const int i1 = (int)fmin(T(kp.nx - 1), floor((cx + Rr - ox) * ih));
   j0 = (int)fmax(T(0), floor((cy - Rr - oy) * ih));
@@ -377,36 +461,58 @@ __device__ __forceinline__ int column_range(const KParams &kp, T cx, T cy, T Rr,
   return (i1 >= i0 && nj > 0) ? (i1 - i0 + 1) * nj : 0;
 }
 
-// Raw sums of one force evaluation, in row order: per site f (3) and U, then
-// the field (3) and its gradient (xx yy zz xy xz yz) at the dipole site.
+// Raw sums of one force evaluation, in row order: the sites' forces (3 each),
+// the field (3) and its gradient (xx yy zz xy xz yz) at the dipole site, then
+// the sites' energies.
+template <int GAS> struct Row {
+  static constexpr int NS = GasShape<GAS>::NS;
+  static constexpr int E = 3 * NS, G = E + 3, U = E + 9, N = U + NS;
+  // the sums that give the forces (a prefix of the row)
+  static constexpr int forces(bool hasq) { return hasq ? U : E; }
+};
 template <typename T, int NS> __device__ __forceinline__ T acc_value(const Acc<T, NS> &acc, int k) {
-  return k < 4 * NS ? (k % 4 == 3 ? acc.Usum(k / 4) : acc.f[k / 4][k % 4])
-                    : (k < 4 * NS + 3 ? acc.E[k - 4 * NS] : acc.G[k - 4 * NS - 3]);
+  return k < 3 * NS ? acc.f[k / 3][k % 3]
+                    : k < 3 * NS + 3 ? acc.E[k - 3 * NS] : k < 3 * NS + 9 ? acc.G[k - 3 * NS - 3] : acc.Usum(k - 3 * NS - 9);
 }
 
-// Site forces and energies from a row of raw sums: the induced-dipole force
-// alpha (E . grad) E and energy -alpha/2 |E|^2 (Force.cpp:483-487) at the
-// dipole site; sites outside the reference grid feel nothing.
+// Site forces (and energies, with WU) from a row of raw sums: the
+// induced-dipole force alpha (E . grad) E and energy -alpha/2 |E|^2
+// (Force.cpp:483-487) at the dipole site; sites outside the reference grid
+// feel nothing.
 template <typename T, int GAS, bool HASQ>
 __device__ __forceinline__ void finish_row(const KParams &kp, const T *row, const bool (&act)[GasShape<GAS>::NS],
-                                           T (&f)[GasShape<GAS>::NS][3], T (&U)[GasShape<GAS>::NS]) {
+                                           T (&f)[GasShape<GAS>::NS][3]) {
   constexpr int NS = GasShape<GAS>::NS;
 #pragma unroll
-  for (int s = 0; s < NS; s++) {
-    f[s][0] = row[4 * s]; f[s][1] = row[4 * s + 1]; f[s][2] = row[4 * s + 2]; U[s] = row[4 * s + 3];
-  }
+  for (int s = 0; s < NS; s++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) f[s][k] = row[3 * s + k];
   if (HASQ && kp.dip_on) {
     constexpr int d = GasShape<GAS>::DIP;
-    const T al = T(kp.alpha);
-    const T *E = row + 4 * NS, *Gr = row + 4 * NS + 3;
+    const T al = kconst<T>(kp).alpha;
+    const T *E = row + Row<GAS>::E, *Gr = row + Row<GAS>::G;
     f[d][0] += al * (E[0] * Gr[0] + E[1] * Gr[3] + E[2] * Gr[4]);
     f[d][1] += al * (E[0] * Gr[3] + E[1] * Gr[1] + E[2] * Gr[5]);
     f[d][2] += al * (E[0] * Gr[4] + E[1] * Gr[5] + E[2] * Gr[2]);
-    U[d] -= T(0.5) * al * (E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
   }
 #pragma unroll
   for (int s = 0; s < NS; s++)
-    if (!act[s]) { f[s][0] = f[s][1] = f[s][2] = U[s] = T(0); }
+    if (!act[s]) f[s][0] = f[s][1] = f[s][2] = T(0);
+}
+// The probe's potential energy from the same row.
+template <typename T, int GAS, bool HASQ>
+__device__ __forceinline__ T finish_energy(const KParams &kp, const T *row, const bool (&act)[GasShape<GAS>::NS]) {
+  constexpr int NS = GasShape<GAS>::NS;
+  T U[NS], u = T(0);
+#pragma unroll
+  for (int s = 0; s < NS; s++) U[s] = row[Row<GAS>::U + s];
+  if (HASQ && kp.dip_on) {
+    const T *E = row + Row<GAS>::E;
+    U[GasShape<GAS>::DIP] -= T(0.5) * kconst<T>(kp).alpha * (E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
+  }
+#pragma unroll
+  for (int s = 0; s < NS; s++) u += act[s] ? U[s] : T(0);
+  return u;
 }
 
 // Site forces and energies of a learned-field step: the exact near sums of
@@ -424,13 +530,13 @@ __device__ __forceinline__ void finish_split(const KParams &kp, const T *row, co
 #pragma unroll
   for (int s = 0; s < NS; s++) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) f[s][k] = row[4 * s + k] + T(ffar[s][k]);
-    U[s] = row[4 * s + 3] + T(ufar[s]);
+    for (int k = 0; k < 3; k++) f[s][k] = row[3 * s + k] + T(ffar[s][k]);
+    U[s] = row[Row<GAS>::U + s] + T(ufar[s]);
   }
   if (HASQ && kp.dip_on) {
     constexpr int d = GasShape<GAS>::DIP;
-    const T al = T(kp.alpha);
-    const T *En = row + 4 * NS, *Gn = row + 4 * NS + 3;  // near E; near Jacobian xx yy zz xy xz yz
+    const T al = kconst<T>(kp).alpha;
+    const T *En = row + Row<GAS>::E, *Gn = row + Row<GAS>::G;  // near E; near Jacobian xx yy zz xy xz yz
     const T E[3] = {En[0] + T(Ef[0]), En[1] + T(Ef[1]), En[2] + T(Ef[2])};
     const T Jt[3][3] = {{Gn[0] + T(Jf[0][0]), Gn[3] + T(Jf[0][1]), Gn[4] + T(Jf[0][2])},
                         {Gn[3] + T(Jf[1][0]), Gn[1] + T(Jf[1][1]), Gn[5] + T(Jf[1][2])},
@@ -451,7 +557,7 @@ __device__ __forceinline__ void finish_split(const KParams &kp, const T *row, co
 //   cen     centre of the sites, off: largest |p_s - cen|
 //   glist   the group's candidate buffer in shared memory, GCAP_PER_LANE * G ints
 constexpr int GCAP_PER_LANE = 8;
-template <typename T, int G, int GAS, bool HASQ, bool SPLIT = false>
+template <typename T, int G, int GAS, bool HASQ, bool SPLIT = false, bool WF = true, bool WU = true>
 __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
                                                  const bool (&act)[GasShape<GAS>::NS], const T (&cen)[3], T off,
                                                  Acc<T, GasShape<GAS>::NS> &acc, uint32_t &visits, int g,
@@ -463,22 +569,23 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
   for (int s = 0; s < NS; s++) any |= act[s];
   if (!any) return;
   uint32_t nvis = 0;
+  const KConst<T> &kc = kconst<T>(kp);
   // candidate sphere around the centre; +1e-3 A so rounding never drops a pair
   // (the near part of the range separation reaches r_out only)
-  const T R = kp.allpairs ? T(INFINITY) : (SPLIT ? T(kp.field.r_out) : T(kp.reach)) + off + T(1e-3);
+  const T R = kp.allpairs ? T(INFINITY) : (SPLIT ? T(kp.field.r_out) : kc.reach) + off + T(1e-3);
   const T cx = cen[0], cy = cen[1], cz = cen[2];
-  const T ex = fmax(fmax(T(kp.bb_lo[0]) - cx, cx - T(kp.bb_hi[0])), T(0));
-  const T ey = fmax(fmax(T(kp.bb_lo[1]) - cy, cy - T(kp.bb_hi[1])), T(0));
-  const T ez = fmax(fmax(T(kp.bb_lo[2]) - cz, cz - T(kp.bb_hi[2])), T(0));
-  const T fx = fmax(cx - T(kp.bb_lo[0]), T(kp.bb_hi[0]) - cx);
-  const T fy = fmax(cy - T(kp.bb_lo[1]), T(kp.bb_hi[1]) - cy);
-  const T fz = fmax(cz - T(kp.bb_lo[2]), T(kp.bb_hi[2]) - cz);
+  const T ex = fmax(fmax(kc.bb_lo[0] - cx, cx - kc.bb_hi[0]), T(0));
+  const T ey = fmax(fmax(kc.bb_lo[1] - cy, cy - kc.bb_hi[1]), T(0));
+  const T ez = fmax(fmax(kc.bb_lo[2] - cz, cz - kc.bb_hi[2]), T(0));
+  const T fx = fmax(cx - kc.bb_lo[0], kc.bb_hi[0] - cx);
+  const T fy = fmax(cy - kc.bb_lo[1], kc.bb_hi[1] - cy);
+  const T fz = fmax(cz - kc.bb_lo[2], kc.bb_hi[2] - cz);
   if ((G > 1 && kp.natoms <= 2 * G) || fx * fx + fy * fy + fz * fz <= R * R) {
     // the whole target inside the reach sphere, or a target of at most two
     // atoms per lane of the group: every atom is a candidate
     for (int ai = g; ai < kp.natoms; ai += G) {
       const Atom<T> a = load_atom<T, GAS>(kp, ai);
-      visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a, acc);
+      visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a, acc);
     }
     if (G == 1 || g == 0) nvis += (uint32_t)kp.natoms;
   } else if (ex * ex + ey * ey + ez * ez <= R * R) {
@@ -492,7 +599,7 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
         nvis += (uint32_t)len;
         for (int ai = b; ai < b + len; ai++) {
           const Atom<T> a = load_atom<T, GAS>(kp, ai);
-          visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a, acc);
+          visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a, acc);
         }
       } else {
         // flatten the G runs of this chunk into the group's list: exclusive scan of run lengths
@@ -511,7 +618,7 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
           const int m = min(GCAP, total - cs);
           for (int t = g; t < m; t += G) {
             const Atom<T> a = load_atom<T, GAS>(kp, glist[t]);
-            visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a, acc);
+            visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a, acc);
           }
           __syncwarp(mask);  // the list is rewritten next
         }
@@ -520,27 +627,6 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
     }
   }
   visits += nvis;
-}
-
-// Site forces of one probe configuration by a group of G lanes; every lane of
-// the group gets the identical result (xor-butterfly sums).  Used by the
-// force-evaluation entry point; the lane pass uses accumulate_group +
-// reduce_group_row instead.
-template <typename T, int G, int GAS, bool HASQ>
-__device__ __forceinline__ void eval_forces(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
-                                         const bool (&act)[GasShape<GAS>::NS], const T (&cen)[3],
-                                         T off, T (&f)[GasShape<GAS>::NS][3],
-                                         T (&U)[GasShape<GAS>::NS], uint32_t &visits, int g,
-                                         unsigned mask, int *glist) {
-  constexpr int NS = GasShape<GAS>::NS;
-  constexpr int NV = 4 * NS + 9;
-  Acc<T, NS> acc;
-  acc.zero();
-  accumulate_group<T, G, GAS, HASQ>(kp, p, act, cen, off, acc, visits, g, mask, glist);
-  T row[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) row[k] = G > 1 ? group_sum<G>(acc_value(acc, k), mask) : acc_value(acc, k);
-  finish_row<T, GAS, HASQ>(kp, row, act, f, U);
 }
 
 // Sum of P values over the 32 lanes of a warp, scattered: a reduce-scatter
@@ -569,34 +655,88 @@ template <int P, typename T> __device__ __forceinline__ void warp_reduce_scatter
 }
 template <int P> constexpr int log2_of() { return P <= 1 ? 0 : 1 + log2_of<P / 2>(); }
 
-// values reduced per force evaluation: per site f (3) and U, then the field
-// (3) and its gradient (6) at the dipole site; padded to a power of two
-template <int GAS> struct RedShape {
-  static constexpr int NV = 4 * GasShape<GAS>::NS + 9;
-  static constexpr int P = NV <= 16 ? 16 : 32;
-};
-// Raw sums of a group's evaluation into row[0..NV) (shared memory).  A full
-// warp reduce-scatters (2P - 1 shuffles, each lane stores the value it ends
-// with); smaller groups sum every value by xor butterfly and lane 0 stores.
-template <typename T, int G, int GAS>
-__device__ __forceinline__ void reduce_group_row(const Acc<T, GasShape<GAS>::NS> &acc, int g, unsigned mask,
-                                                 T *row) {
-  constexpr int NV = RedShape<GAS>::NV;
-  if constexpr (G == 32) {
-    constexpr int P = RedShape<GAS>::P;
+// Sums of N values over a warp, into row[0..N) (shared memory, or per-thread
+// storage when every lane calls with its own): reduce-scatters of power-of-two
+// size, split or padded, whichever takes fewer shuffles (18 values: 16 + 2 in
+// 21, not 32 in 31).  Every value's sum runs over the same tree (lane offsets
+// 16, 8, 4, 2, 1) however the values are grouped.
+constexpr int rs_cost(int P) { return P - 1 + (P <= 1 ? 5 : P <= 2 ? 4 : P <= 4 ? 3 : P <= 8 ? 2 : P <= 16 ? 1 : 0); }
+constexpr int pow2_up(int n) { int p = 1; while (p < n) p *= 2; return p; }
+constexpr int pow2_down(int n) { int p = 1; while (2 * p <= n) p *= 2; return p; }
+constexpr int rs_best(int n) {
+  return n <= 0 ? 0
+                : pow2_up(n) <= 32 && (pow2_up(n) == n || rs_cost(pow2_up(n)) <= rs_cost(pow2_down(n)) + rs_best(n - pow2_down(n)))
+                      ? rs_cost(pow2_up(n))
+                      : rs_cost(pow2_down(n)) + rs_best(n - pow2_down(n));
+}
+template <int N, typename T, typename V> __device__ __forceinline__ void warp_sum_rows(const V &value, int base, int lane, T *row) {
+  if constexpr (N > 0) {
+    constexpr int UP = pow2_up(N), DN = pow2_down(N);
+    constexpr bool PAD = UP <= 32 && (UP == N || rs_cost(UP) <= rs_cost(DN) + rs_best(N - DN));
+    constexpr int P = PAD ? UP : DN;
     T v[P];
 #pragma unroll
-    for (int k = 0; k < P; k++) v[k] = k < NV ? acc_value(acc, k) : T(0);
-    warp_reduce_scatter<P>(v, g);
+    for (int k = 0; k < P; k++) v[k] = k < N ? value(base + k) : T(0);
+    warp_reduce_scatter<P>(v, lane);
     constexpr int SH = 5 - log2_of<P>();
-    if ((g & ((1 << SH) - 1)) == 0 && (g >> SH) < NV) row[g >> SH] = v[0];
+    if ((lane & ((1 << SH) - 1)) == 0 && (lane >> SH) < N) row[base + (lane >> SH)] = v[0];
+    warp_sum_rows<N - P>(value, base + P, lane, row);
+  }
+}
+
+// values reduced per force evaluation with energies: the whole row, padded to a power of two
+template <int GAS> struct RedShape {
+  static constexpr int NV = Row<GAS>::N;
+  static constexpr int P = NV <= 16 ? 16 : 32;
+};
+// Raw sums k0 <= k < k1 of a group's evaluation into row[k0..k1) (shared
+// memory).  A full warp reduce-scatters; smaller groups sum every value by
+// xor butterfly and lane 0 stores.
+template <typename T, int G, int GAS, int K0, int K1>
+__device__ __forceinline__ void reduce_group_row(const Acc<T, GasShape<GAS>::NS> &acc, int g, unsigned mask,
+                                                 T *row) {
+  if constexpr (G == 32) {
+    warp_sum_rows<K1 - K0, T>([&](int k) { return acc_value(acc, k); }, K0, g, row);
   } else {
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
+    for (int k = K0; k < K1; k++) {
       const T x = G > 1 ? group_sum<G>(acc_value(acc, k), mask) : acc_value(acc, k);
       if (g == 0) row[k] = x;
     }
   }
+}
+
+// The energies of one probe configuration (row[U..U + NS)), in the order of
+// its force sums.  Out of line: a trajectory needs it twice.
+template <typename T, int GAS> struct ProbeSites {
+  T p[GasShape<GAS>::NS][3];
+  bool act[GasShape<GAS>::NS];
+};
+template <typename T, int G, int GAS, bool HASQ>
+__device__ __noinline__ void group_energy(const KParams *__restrict__ kpg, const ProbeSites<T, GAS> ps, T off, int g,
+                                          unsigned mask, int *glist, T *row) {
+  Acc<T, GasShape<GAS>::NS> acc;
+  acc.zero();
+  uint32_t nv = 0;
+  const T cen[3] = {ps.p[Sites<GAS>::cs][0], ps.p[Sites<GAS>::cs][1], ps.p[Sites<GAS>::cs][2]};
+  accumulate_group<T, G, GAS, HASQ, false, false, true>(*kpg, ps.p, ps.act, cen, off, acc, nv, g, mask, glist);
+  reduce_group_row<T, G, GAS, Row<GAS>::U, Row<GAS>::N>(acc, g, mask, row);
+}
+
+// The raw sums (and with WU the energies) of one probe configuration by a
+// group of G lanes, every lane of the group with the identical row
+// (xor-butterfly sums): the force-evaluation entry point, and the lane pass
+// with one lane per force evaluation.
+template <typename T, int G, int GAS, bool HASQ, bool WU>
+__device__ __forceinline__ void eval_row(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
+                                         const bool (&act)[GasShape<GAS>::NS], const T (&cen)[3], T off, T *row,
+                                         uint32_t &visits, int g, unsigned mask, int *glist) {
+  Acc<T, GasShape<GAS>::NS> acc;
+  acc.zero();
+  accumulate_group<T, G, GAS, HASQ, false, true, WU>(kp, p, act, cen, off, acc, visits, g, mask, glist);
+#pragma unroll
+  for (int k = 0; k < (WU ? Row<GAS>::N : Row<GAS>::forces(HASQ)); k++)
+    row[k] = G > 1 ? group_sum<G>(acc_value(acc, k), mask) : acc_value(acc, k);
 }
 
 constexpr int LCAP = 2048;  // least candidate-list entries kept in shared memory per CTA (the
@@ -635,15 +775,16 @@ __device__ __forceinline__ void visit_list(const KParams &kp, const T (&p)[GasSh
                                            const bool (&act)[GasShape<GAS>::NS], const int *list, int m, int tid,
                                            Acc<T, GasShape<GAS>::NS> &acc) {
   int t = tid;
+  constexpr bool PF = sizeof(T) == 4 && GAS == GAS_CO2;  // see visit_atom's DIPF
   for (; t + NT < m; t += 2 * NT) {
     const Atom<T> a1 = load_atom<T, GAS>(kp, list ? list[t] : t);
     const Atom<T> a2 = load_atom<T, GAS>(kp, list ? list[t + NT] : t + NT);
-    visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a1, acc);
-    visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a2, acc);
+    visit_atom<T, GAS, HASQ, SPLIT, true, true, PF>(kp, p, act, a1, acc);
+    visit_atom<T, GAS, HASQ, SPLIT, true, true, PF>(kp, p, act, a2, acc);
   }
   if (t < m) {
     const Atom<T> a1 = load_atom<T, GAS>(kp, list ? list[t] : t);
-    visit_atom<T, GAS, HASQ, SPLIT>(kp, p, act, a1, acc);
+    visit_atom<T, GAS, HASQ, SPLIT, true, true, PF && NT != 32>(kp, p, act, a1, acc);
   }
 }
 
@@ -651,10 +792,6 @@ __device__ __forceinline__ void visit_list(const KParams &kp, const T (&p)[GasSh
 // flattened chunk by chunk.  Kept out of line (large targets only) and given
 // copies of the probe, so the common step's code stays compact and its
 // registers never need an address.
-template <typename T, int GAS> struct ProbeSites {
-  T p[GasShape<GAS>::NS][3];
-  bool act[GasShape<GAS>::NS];
-};
 template <typename T, int NT, int GAS, bool HASQ, bool SPLIT = false>
 __device__ __noinline__ Acc<T, GasShape<GAS>::NS> chunked_visits(const KParams *__restrict__ kpg,
                                                                  const ProbeSites<T, GAS> ps, T cx, T cy, T cz,
@@ -714,8 +851,8 @@ __device__ __noinline__ Acc<T, GasShape<GAS>::NS> chunked_visits(const KParams *
 template <typename T, int NT, int GAS, bool HASQ, bool SPLIT = false>
 __device__ __forceinline__ void eval_forces_block(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
                                                   const bool (&act)[GasShape<GAS>::NS], const T (&cen)[3],
-                                                  T off, T (&f)[GasShape<GAS>::NS][3],
-                                                  T (&U)[GasShape<GAS>::NS], uint32_t &visits, int tid,
+                                                  T off, T (&f)[GasShape<GAS>::NS][3], T &upot,
+                                                  uint32_t &visits, int tid,
                                                   int *sm_list, int lcap, int *sm_wsum, T *sm_red, int &list_n,
                                                   T (&list_c)[3], const KParams *__restrict__ kpg,
                                                   T *raw = nullptr) {
@@ -724,6 +861,7 @@ __device__ __forceinline__ void eval_forces_block(const KParams &kp, const T (&p
   constexpr int NV = RedShape<GAS>::NV;
   constexpr int P = RedShape<GAS>::P;
   const int lane = tid & 31, w = tid >> 5;
+  const KConst<T> &kc = kconst<T>(kp);
   Acc<T, NS> acc;
   acc.zero();
   bool any = false;
@@ -731,14 +869,14 @@ __device__ __forceinline__ void eval_forces_block(const KParams &kp, const T (&p
   for (int s = 0; s < NS; s++) any |= act[s];
   uint32_t nvis = 0;
   if (any) {
-    const T R = kp.allpairs ? T(INFINITY) : (SPLIT ? T(kp.field.r_out) : T(kp.reach)) + off + T(1e-3);
+    const T R = kp.allpairs ? T(INFINITY) : (SPLIT ? T(kp.field.r_out) : kc.reach) + off + T(1e-3);
     const T cx = cen[0], cy = cen[1], cz = cen[2];
-    const T ex = fmax(fmax(T(kp.bb_lo[0]) - cx, cx - T(kp.bb_hi[0])), T(0));
-    const T ey = fmax(fmax(T(kp.bb_lo[1]) - cy, cy - T(kp.bb_hi[1])), T(0));
-    const T ez = fmax(fmax(T(kp.bb_lo[2]) - cz, cz - T(kp.bb_hi[2])), T(0));
-    const T fx = fmax(cx - T(kp.bb_lo[0]), T(kp.bb_hi[0]) - cx);
-    const T fy = fmax(cy - T(kp.bb_lo[1]), T(kp.bb_hi[1]) - cy);
-    const T fz = fmax(cz - T(kp.bb_lo[2]), T(kp.bb_hi[2]) - cz);
+    const T ex = fmax(fmax(kc.bb_lo[0] - cx, cx - kc.bb_hi[0]), T(0));
+    const T ey = fmax(fmax(kc.bb_lo[1] - cy, cy - kc.bb_hi[1]), T(0));
+    const T ez = fmax(fmax(kc.bb_lo[2] - cz, cz - kc.bb_hi[2]), T(0));
+    const T fx = fmax(cx - kc.bb_lo[0], kc.bb_hi[0] - cx);
+    const T fy = fmax(cy - kc.bb_lo[1], kc.bb_hi[1] - cy);
+    const T fz = fmax(cz - kc.bb_lo[2], kc.bb_hi[2] - cz);
     const int *lst = nullptr;  // candidates: atoms 0..m (nullptr) or lst[0..m)
     int m = 0;
     if (kp.natoms <= 2 * NT || fx * fx + fy * fy + fz * fz <= R * R) {
@@ -788,15 +926,7 @@ __device__ __forceinline__ void eval_forces_block(const KParams &kp, const T (&p
   // reduce-scatter per warp, then the warps in a fixed order
   T v[P];
 #pragma unroll
-  for (int s = 0; s < NS; s++) {
-    v[4 * s] = acc.f[s][0]; v[4 * s + 1] = acc.f[s][1]; v[4 * s + 2] = acc.f[s][2]; v[4 * s + 3] = acc.Usum(s);
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++) v[4 * NS + k] = acc.E[k];
-#pragma unroll
-  for (int k = 0; k < 6; k++) v[4 * NS + 3 + k] = acc.G[k];
-#pragma unroll
-  for (int k = NV; k < P; k++) v[k] = T(0);
+  for (int k = 0; k < P; k++) v[k] = k < NV ? acc_value(acc, k) : T(0);
   warp_reduce_scatter<P>(v, lane);
   constexpr int SH = 5 - log2_of<P>();  // lanes per value index = 1 << SH
   T out[NV];
@@ -821,22 +951,8 @@ __device__ __forceinline__ void eval_forces_block(const KParams &kp, const T (&p
     visits += nvis;
     return;
   }
-#pragma unroll
-  for (int s = 0; s < NS; s++) {
-    f[s][0] = out[4 * s]; f[s][1] = out[4 * s + 1]; f[s][2] = out[4 * s + 2]; U[s] = out[4 * s + 3];
-  }
-  if (HASQ && kp.dip_on) {
-    constexpr int d = GasShape<GAS>::DIP;
-    const T al = T(kp.alpha);
-    const T *E = out + 4 * NS, *Gr = out + 4 * NS + 3;
-    f[d][0] += al * (E[0] * Gr[0] + E[1] * Gr[3] + E[2] * Gr[4]);
-    f[d][1] += al * (E[0] * Gr[3] + E[1] * Gr[1] + E[2] * Gr[5]);
-    f[d][2] += al * (E[0] * Gr[4] + E[1] * Gr[5] + E[2] * Gr[2]);
-    U[d] -= T(0.5) * al * (E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
-  }
-#pragma unroll
-  for (int s = 0; s < NS; s++)
-    if (!act[s]) { f[s][0] = f[s][1] = f[s][2] = U[s] = T(0); }
+  finish_row<T, GAS, HASQ>(kp, out, act, f);
+  upot = finish_energy<T, GAS, HASQ>(kp, out, act);
   visits += nvis;
 }
 
@@ -969,8 +1085,9 @@ __device__ __forceinline__ double one_minus_cos(const double vi[3], const T vf[3
   }
 }
 template <typename T> __device__ __forceinline__ bool outside_box(const KParams &kp, const T r[3]) {
-  if (fabs(r[0]) >= T(kp.lx) || fabs(r[1]) >= T(kp.ly) || fabs(r[2]) >= T(kp.lz)) return true;
-  const T ux = r[0] * T(kp.inv_a), uy = r[1] * T(kp.inv_b), uz = r[2] * T(kp.inv_c);
+  const KConst<T> &kc = kconst<T>(kp);
+  if (fabs(r[0]) >= kc.lx || fabs(r[1]) >= kc.ly || fabs(r[2]) >= kc.lz) return true;
+  const T ux = r[0] * kc.inv_a, uy = r[1] * kc.inv_b, uz = r[2] * kc.inv_c;
   return ux * ux + uy * uy + uz * uz > T(1);
 }
 
@@ -1029,12 +1146,6 @@ template <typename T> struct LaneState {
   unsigned long long j;
 };
 
-template <int GAS> struct Sites {
-  static constexpr int NS = GasShape<GAS>::NS;
-  static constexpr int pa = 0, pb = GAS == GAS_CO2 ? 2 : 1, pc = GAS == GAS_CO2 ? 1 : 2;
-  static constexpr int cs = GAS == GAS_ATOM ? 0 : pc;  // reference point of the reach sphere
-};
-
 template <typename T, int GAS>
 __device__ __forceinline__ void site_positions(const LaneState<T> &L, T (&p)[GasShape<GAS>::NS][3]) {
   using S = Sites<GAS>;
@@ -1068,29 +1179,32 @@ template <typename T, int GAS>
 __device__ __forceinline__ bool probe_near(const KParams &kp, const T (&p)[GasShape<GAS>::NS][3],
                                            unsigned &actbits) {
   using S = Sites<GAS>;
-  actbits = 0;
+  const KConst<T> &kc = kconst<T>(kp);
+  const T off = site_offset<T, GAS>(p);
+  actbits = (1u << S::NS) - 1u;
+  // well inside the reference grid (nearly always) every site is; near its faces, site by site
+  if (!(fabs(p[S::cs][0]) + off < kc.ref_lim[0] && fabs(p[S::cs][1]) + off < kc.ref_lim[1] &&
+        fabs(p[S::cs][2]) + off < kc.ref_lim[2])) {
+    actbits = 0;
 #pragma unroll
-  for (int s = 0; s < S::NS; s++)
-    if (ref_inside(kp, p[s][0], p[s][1], p[s][2])) actbits |= 1u << s;
-  const T R = (kp.allpairs ? T(INFINITY) : T(kp.reach) + T(1e-3)) + site_offset<T, GAS>(p);
-  const T ex = fmax(fmax(T(kp.bb_lo[0]) - p[S::cs][0], p[S::cs][0] - T(kp.bb_hi[0])), T(0));
-  const T ey = fmax(fmax(T(kp.bb_lo[1]) - p[S::cs][1], p[S::cs][1] - T(kp.bb_hi[1])), T(0));
-  const T ez = fmax(fmax(T(kp.bb_lo[2]) - p[S::cs][2], p[S::cs][2] - T(kp.bb_hi[2])), T(0));
+    for (int s = 0; s < S::NS; s++)
+      if (ref_inside(kp, p[s][0], p[s][1], p[s][2])) actbits |= 1u << s;
+  }
+  const T R = (kp.allpairs ? T(INFINITY) : kc.reach + T(1e-3)) + off;
+  const T ex = fmax(fmax(kc.bb_lo[0] - p[S::cs][0], p[S::cs][0] - kc.bb_hi[0]), T(0));
+  const T ey = fmax(fmax(kc.bb_lo[1] - p[S::cs][1], p[S::cs][1] - kc.bb_hi[1]), T(0));
+  const T ez = fmax(fmax(kc.bb_lo[2] - p[S::cs][2], p[S::cs][2] - kc.bb_hi[2]), T(0));
   return actbits != 0 && ex * ex + ey * ey + ez * ez <= R * R;
 }
 
 // pair forces from the site forces: N2 splits the central charge half/half
 // (System.cpp:736-739); CO2 redistributes the carbon force (Ciccotti,
-// System.cpp:1154-1158); an atom keeps its own force.  Also sums U.
+// System.cpp:1154-1158); an atom keeps its own force.
 template <typename T, int GAS>
 __device__ __forceinline__ void absorb_forces(const KParams &kp, const T (&fs)[GasShape<GAS>::NS][3],
-                                              const T (&Us)[GasShape<GAS>::NS], LaneState<T> &L) {
-  T u = T(0);
-#pragma unroll
-  for (int s = 0; s < GasShape<GAS>::NS; s++) u += Us[s];
-  L.U = u;
+                                              LaneState<T> &L) {
   if constexpr (GAS == GAS_CO2) {
-    const T M = T(kp.gas_mass), m2M = T(kp.gas_m[1]) / M, m0M = T(kp.gas_m[0]) / M;
+    const T m2M = kconst<T>(kp).m2M, m0M = kconst<T>(kp).m0M;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       L.f1[k] = (T(1) - T(0.5) * m2M) * fs[0][k] + m0M * fs[1][k] - T(0.5) * m2M * fs[2][k];
@@ -1173,9 +1287,10 @@ __device__ __noinline__ double lane_chi(const KParams *__restrict__ kpg, unsigne
 template <typename T, int GAS>
 __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
   using S = Sites<GAS>;
-  const T dt = L.dt, kconv = T(KCALMOLANGAMU_TO_ANGFS2);
+  const KConst<T> &kc = kconst<T>(kp);
+  const T dt = L.dt;
   if constexpr (GAS == GAS_ATOM) {
-    const T kick = dt * T(kp.half_kconv_over_m1);
+    const T kick = dt * kc.half_kconv_over_m1;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       L.v1[k] += kick * L.f1[k];
@@ -1189,8 +1304,8 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
     for (int k = 0; k < 3; k++) L.rold[k] = L.r1[k];
   } else {
     // constrained Verlet, first half (System.cpp:1700-1739)
-    const T d2 = T(kp.d_bond * kp.d_bond);
-    const T ka = dt * T(kp.half_kconv_over_m1), kb = dt * T(kp.half_kconv_over_m2);
+    const T d2 = sizeof(T) == 4 ? kc.d2 : T(kp.d_bond * kp.d_bond);
+    const T ka = dt * kc.half_kconv_over_m1, kb = dt * kc.half_kconv_over_m2;
     T vci[3], vcj[3], rij[3], rcij[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -1203,9 +1318,9 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
     T det = rr * rr - r2ij * (rc2ij - d2);
     if (det < T(0)) det = T(0);
     const T lam = Real<T>::div(rr - Real<T>::sq(det), r2ij);
-    const T cpos = T(kp.mu12_over_m1) * lam;  // the reference uses mi for both atoms (:1735-1736)
+    const T cpos = kc.mu12_over_m1 * lam;  // the reference uses mi for both atoms (:1735-1736)
     const T inv_dt = Real<T>::div(T(1), dt);
-    const T ca = cpos * inv_dt, cb = T(kp.mu12_over_m2) * lam * inv_dt;
+    const T ca = cpos * inv_dt, cb = kc.mu12_over_m2 * lam * inv_dt;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       L.v1[k] = vci[k] - ca * rij[k];
@@ -1230,22 +1345,28 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
 
 enum : int { S_CONTINUE = 0, S_RETRY_ANGLE = 1, S_RETRY_ENERGY = 2, S_SCATTER = 3, S_CAPPED = 4 };
 
+// Whether the step that first_half has begun ends outside the box or the
+// ellipsoid: the second half moves no position, so this is known before the
+// forces are (and with it whether the step needs the potential energy).
+template <typename T> __device__ __forceinline__ bool step_leaves(const KParams &kp, const LaneState<T> &L) {
+  return outside_box(kp, L.rold);  // first_half left the (centre) position there
+}
+
 // Second half of a step and the exit tests (System.cpp:441-506, 835-940,
-// 1268-1387).  vc receives the centre-of-mass velocity for chi.
+// 1268-1387).  out = step_leaves(); L.U is read only when it is set.  The
+// centre-of-mass velocity for chi is exit_velocity's.
 template <typename T, int GAS>
-__device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, T vc[3]) {
+__device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, bool out) {
   using S = Sites<GAS>;
-  const T dt = L.dt, kconv = T(KCALMOLANGAMU_TO_ANGFS2), ke = T(AMUANGFS2_TO_KCAL_MOL);
-  T rc[3], ek;
+  const KConst<T> &kc = kconst<T>(kp);
+  const T dt = L.dt, ke = T(AMUANGFS2_TO_KCAL_MOL);
   if constexpr (GAS == GAS_ATOM) {
-    const T kick = dt * T(kp.half_kconv_over_m1);
+    const T kick = dt * kc.half_kconv_over_m1;
 #pragma unroll
-    for (int k = 0; k < 3; k++) { L.v1[k] += kick * L.f1[k]; vc[k] = L.v1[k]; rc[k] = L.r1[k]; }
-    ek = T(0.5) * T(kp.mu) * dot3(L.v1, L.v1) * ke;
+    for (int k = 0; k < 3; k++) L.v1[k] += kick * L.f1[k];
   } else {
     // RATTLE velocity correction (System.cpp:1741-1767)
-    const T ma = T(kp.gas_m[S::pa]), mb = T(kp.gas_m[S::pb]);
-    const T ka = dt * T(kp.half_kconv_over_m1), kb = dt * T(kp.half_kconv_over_m2);
+    const T ka = dt * kc.half_kconv_over_m1, kb = dt * kc.half_kconv_over_m2;
     T vci[3], vcj[3], rij[3], vcij[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -1254,28 +1375,39 @@ __device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, T
       rij[k] = L.r1[k] - L.r2[k];
       vcij[k] = vci[k] - vcj[k];
     }
-    const T lam = Real<T>::div(T(kp.mu12) * dot3(rij, vcij), dot3(rij, rij));
-    const T la = lam * T(kp.inv_m1), lb = lam * T(kp.inv_m2);
+    const T lam = Real<T>::div(kc.mu12 * dot3(rij, vcij), dot3(rij, rij));
+    const T la = lam * kc.inv_m1, lb = lam * kc.inv_m2;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       L.v1[k] = vci[k] - la * rij[k];
       L.v2[k] = vcj[k] + lb * rij[k];
-      vc[k] = T(0.5) * (L.v1[k] + L.v2[k]);
-      rc[k] = T(0.5) * (L.r1[k] + L.r2[k]);
     }
-    // N2: the two N atoms (System.cpp:890-896); CO2: all sites, carbon at vcm (:1333-1339)
-    ek = T(0.5) * ma * dot3(L.v1, L.v1) * ke + T(0.5) * mb * dot3(L.v2, L.v2) * ke;
-    if (GAS == GAS_CO2) ek += T(0.5) * T(kp.gas_m[S::pc]) * dot3(vc, vc) * ke;
   }
   L.stepcount++;
   L.nsteps++;
   if (L.dtheta > T(1.5 * PI_D)) return S_RETRY_ANGLE;
-  if (outside_box(kp, rc)) {
+  if (out) {
+    T ek;
+    if constexpr (GAS == GAS_ATOM) {
+      ek = T(0.5) * kc.mu * dot3(L.v1, L.v1) * ke;
+    } else {
+      // N2: the two N atoms (System.cpp:890-896); CO2: all sites, carbon at vcm (:1333-1339)
+      const T ma = kc.gas_m[S::pa], mb = kc.gas_m[S::pb];
+      ek = T(0.5) * ma * dot3(L.v1, L.v1) * ke + T(0.5) * mb * dot3(L.v2, L.v2) * ke;
+      if (GAS == GAS_CO2) {
+        const T vc[3] = {T(0.5) * (L.v1[0] + L.v2[0]), T(0.5) * (L.v1[1] + L.v2[1]), T(0.5) * (L.v1[2] + L.v2[2])};
+        ek += T(0.5) * kc.gas_m[S::pc] * dot3(vc, vc) * ke;
+      }
+    }
     const double E = (double)L.U + (double)ek;
     const double dE = fabs((E - (double)L.Ei) / (double)L.Ei) * 100.0;
     return dE > kp.etol ? S_RETRY_ENERGY : S_SCATTER;
   }
   return L.stepcount >= kp.max_steps ? S_CAPPED : S_CONTINUE;
+}
+// Component k of the centre-of-mass velocity.
+template <typename T, int GAS> __device__ __forceinline__ T exit_velocity(const LaneState<T> &L, int k) {
+  return GAS == GAS_ATOM ? L.v1[k] : T(0.5) * (L.v1[k] + L.v2[k]);
 }
 
 // Result of one trajectory.
@@ -1314,7 +1446,8 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
   static_assert(!SURR || (sizeof(T) == 4 && !BATCH), "the learned field runs in FP32 single-ion launches");
   constexpr int NSUB = 32 / G;
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int NV = RedShape<GAS>::NV;
+  constexpr int NV = Row<GAS>::N, NF = Row<GAS>::forces(HASQ);
+  constexpr unsigned WANT_U = 1u << 8;  // sm_act: the probe's energy is wanted too
   __shared__ T sm_pos[BLOCK][NS][3];
   __shared__ T sm_row[BLOCK][NV];
   __shared__ uint32_t sm_vis[BLOCK];
@@ -1364,6 +1497,7 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
       if (!I.hit) { write_result(K, L, 0, 0.0, blk); continue; }
       load_init<T, GAS>(L, I);
       L.Ei = I.ek;  // completed with the initial potential energy by the first force phase
+      L.U = T(0);
       L.tries = 0;
       L.maxTries = 8;
       L.dt = T(K.dt);
@@ -1372,7 +1506,9 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
     }
   };
 
-  grab();
+  // few trajectories: fewer lanes of each warp take one, so that all warps
+  // have work (a warp evaluates its probes' forces one after another)
+  if (lane < kp.lane_width) grab();
   unsigned it = 0;
   for (;;) {
     if ((++it & 127u) == 0) {  // watchdog, one answer per warp
@@ -1392,14 +1528,20 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
     }
     const KParams &K = ion_params<BATCH>(kp, L.ion);  // this lane's ion
 
-    if (L.mode == M_STEP) first_half<T, GAS>(K, L);
+    bool out = false;
+    if (L.mode == M_STEP) {
+      first_half<T, GAS>(K, L);
+      out = step_leaves(K, L);
+    }
 
     // ---- force phase
     bool near = false, surr = false;
+    const bool want_u = L.mode == M_INIT || out;  // the energy test's two ends
     unsigned actbits = 0;
-    T fs[NS][3], Us[NS];
+    T fs[NS][3];
     T p[NS][3];
     if (L.mode != M_IDLE) {
+      if (want_u) L.U = T(0);
       site_positions<T, GAS>(L, p);
       near = probe_near<T, GAS>(K, p, actbits);
       if constexpr (SURR) {
@@ -1415,15 +1557,32 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
           bool act[NS];
 #pragma unroll
           for (int s = 0; s < NS; s++) act[s] = (actbits >> s) & 1u;
-          if (!surr)
-            eval_forces<T, 1, GAS, HASQ>(K, p, act, p[S::cs], site_offset<T, GAS>(p), fs, Us, L.nvis, 0,
-                                         1u << lane, nullptr);
+          if (!surr) {
+            T row[NV];
+            eval_row<T, 1, GAS, HASQ, false>(K, p, act, p[S::cs], site_offset<T, GAS>(p), row, L.nvis, 0, 1u << lane,
+                                             nullptr);
+            finish_row<T, GAS, HASQ>(K, row, act, fs);
+            if (want_u) {
+              ProbeSites<T, GAS> ps;
+#pragma unroll
+              for (int s = 0; s < NS; s++) {
+                ps.act[s] = act[s];
+#pragma unroll
+                for (int k = 0; k < 3; k++) ps.p[s][k] = p[s][k];
+              }
+              group_energy<T, 1, GAS, HASQ>(ion_params_ptr<BATCH>(kp, kpg, L.ion), ps, site_offset<T, GAS>(p), 0,
+                                            1u << lane, nullptr, sm_row[threadIdx.x]);
+#pragma unroll
+              for (int s = 0; s < NS; s++) row[Row<GAS>::U + s] = sm_row[threadIdx.x][Row<GAS>::U + s];
+              L.U = finish_energy<T, GAS, HASQ>(K, row, act);
+            }
+          }
         } else {
 #pragma unroll
           for (int s = 0; s < NS; s++)
 #pragma unroll
             for (int k = 0; k < 3; k++) sm_pos[threadIdx.x][s][k] = p[s][k];
-          sm_act[threadIdx.x] = actbits;
+          sm_act[threadIdx.x] = actbits | (want_u ? WANT_U : 0u);
           if constexpr (BATCH) sm_ion[threadIdx.x] = L.ion;
         }
       }
@@ -1447,17 +1606,30 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
         Acc<T, NS> acc;
         acc.zero();
         const KParams &Kt = ion_params<BATCH>(kp, BATCH ? sm_ion[t] : 0u);  // the probe's ion
-        accumulate_group<T, G, GAS, HASQ>(Kt, P, act, P[S::cs], site_offset<T, GAS>(P), acc, nv, g, gmask,
-                                          sm_glist + (wbase + sub * G) * GCAP_PER_LANE);
-        reduce_group_row<T, G, GAS>(acc, g, gmask, sm_row[t]);
+        int *const glist = sm_glist + (wbase + sub * G) * GCAP_PER_LANE;
+        accumulate_group<T, G, GAS, HASQ, false, true, false>(Kt, P, act, P[S::cs], site_offset<T, GAS>(P), acc, nv,
+                                                              g, gmask, glist);
+        reduce_group_row<T, G, GAS, 0, NF>(acc, g, gmask, sm_row[t]);
         if (g == 0) sm_vis[t] = nv;
+        if (ab & WANT_U) {  // group-uniform
+          ProbeSites<T, GAS> ps;
+#pragma unroll
+          for (int s = 0; s < NS; s++) {
+            ps.act[s] = act[s];
+#pragma unroll
+            for (int k = 0; k < 3; k++) ps.p[s][k] = P[s][k];
+          }
+          group_energy<T, G, GAS, HASQ>(ion_params_ptr<BATCH>(kp, kpg, BATCH ? sm_ion[t] : 0u), ps,
+                                        site_offset<T, GAS>(P), g, gmask, glist, sm_row[t]);
+        }
       }
       __syncwarp();
       if (near && !surr) {  // the probe's own lane finishes its forces from the raw sums
         bool act[NS];
 #pragma unroll
         for (int s = 0; s < NS; s++) act[s] = (actbits >> s) & 1u;
-        finish_row<T, GAS, HASQ>(K, sm_row[threadIdx.x], act, fs, Us);
+        finish_row<T, GAS, HASQ>(K, sm_row[threadIdx.x], act, fs);
+        if (want_u) L.U = finish_energy<T, GAS, HASQ>(K, sm_row[threadIdx.x], act);
         L.nvis += sm_vis[threadIdx.x];
       }
     }
@@ -1499,7 +1671,7 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
           acc.zero();
           accumulate_group<T, G, GAS, HASQ, true>(kp, P, at, P[S::cs], site_offset<T, GAS>(P), acc, nv, g, gmask,
                                                   sm_glist + (wbase + sub * G) * GCAP_PER_LANE);
-          reduce_group_row<T, G, GAS>(acc, g, gmask, sm_row[t]);
+          reduce_group_row<T, G, GAS, 0, NV>(acc, g, gmask, sm_row[t]);
           if (g == 0) sm_vis[t] = nv;
         }
         __syncwarp();
@@ -1544,14 +1716,20 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
           break;
         }
       }
-      if (surr) finish_split<T, GAS, HASQ>(K, raw, ufar, ffar, Ef, Jf, act, fs, Us);
+      if (surr) {
+        T Us[NS];
+        finish_split<T, GAS, HASQ>(K, raw, ufar, ffar, Ef, Jf, act, fs, Us);
+        L.U = T(0);
+#pragma unroll
+        for (int s = 0; s < NS; s++) L.U += Us[s];
+      }
     }
     if (L.mode == M_IDLE) continue;
     if (!near) {
 #pragma unroll
-      for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = Us[s] = T(0);
+      for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = T(0);
     }
-    absorb_forces<T, GAS>(K, fs, Us, L);
+    absorb_forces<T, GAS>(K, fs, L);
 
     // ---- second half, exit tests, retries, parking
     if (L.mode == M_INIT) {
@@ -1560,10 +1738,10 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
     } else if (L.mode == M_RESTART) {
       L.mode = M_STEP;
     } else {
-      T vc[3];
-      const int r = second_half<T, GAS>(K, L, vc);
+      const int r = second_half<T, GAS>(K, L, out);
       if (r == S_SCATTER) {
-        write_result(K, L, 1, lane_chi<T, GAS>(ion_params_ptr<BATCH>(kp, kpg, L.ion), L.j, vc[0], vc[1], vc[2]), blk);
+        write_result(K, L, 1, lane_chi<T, GAS>(ion_params_ptr<BATCH>(kp, kpg, L.ion), L.j, exit_velocity<T, GAS>(L, 0),
+                                               exit_velocity<T, GAS>(L, 1), exit_velocity<T, GAS>(L, 2)), blk);
         grab();
       } else if (r == S_CAPPED) {
         write_result(K, L, 3, 0.0, blk);
@@ -1752,8 +1930,13 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
         }
       }
       if (r == S_CONTINUE) {
-        if (L.mode == M_STEP) first_half<T, GAS>(K, L);
-        T p[NS][3], fs[NS][3], Us[NS];
+        bool out = false;
+        if (L.mode == M_STEP) {
+          first_half<T, GAS>(K, L);
+          out = step_leaves(K, L);
+        }
+        T p[NS][3], fs[NS][3];
+        L.U = T(0);
         site_positions<T, GAS>(L, p);
         unsigned actbits;
         if (probe_near<T, GAS>(K, p, actbits)) {
@@ -1771,7 +1954,8 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
             if constexpr (SURR) {
               // the switched exact sums over the atoms within r_out ...
               T raw[RedShape<GAS>::NV];
-              eval_forces_block<T, NT, GAS, HASQ, true>(K, p, act, p[S::cs], site_offset<T, GAS>(p), fs, Us, L.nvis,
+              T none;
+              eval_forces_block<T, NT, GAS, HASQ, true>(K, p, act, p[S::cs], site_offset<T, GAS>(p), fs, none, L.nvis,
                                                         tid, sm_list + kp.lcap, LCAP, sm_wsum, sm_red[red], near_n, near_c, Kg, raw);
               red ^= 1;
               // ... plus the far parts from the network, one warp per site
@@ -1804,24 +1988,28 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
                 for (int b = 0; b < 3; b++) Jf[a][b] = ds >= 0 ? -sm_site[ds < NS ? ds : 0][4 * (1 + a) + 1 + b] : 0.f;
               }
               __syncthreads();
+              T Us[NS];
               finish_split<T, GAS, HASQ>(K, raw, ufar, ffar, Ef, Jf, act, fs, Us);
+#pragma unroll
+              for (int s = 0; s < NS; s++) L.U += Us[s];
             }
           } else {
-            eval_forces_block<T, NT, GAS, HASQ>(K, p, act, p[S::cs], site_offset<T, GAS>(p), fs, Us, L.nvis,
+            eval_forces_block<T, NT, GAS, HASQ>(K, p, act, p[S::cs], site_offset<T, GAS>(p), fs, L.U, L.nvis,
                                                   tid, sm_list, kp.lcap, sm_wsum, sm_red[red], list_n, list_c, Kg);
             red ^= 1;
           }
         } else {
 #pragma unroll
-          for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = Us[s] = T(0);
+          for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = T(0);
         }
-        absorb_forces<T, GAS>(K, fs, Us, L);
+        absorb_forces<T, GAS>(K, fs, L);
         if (L.mode == M_INIT) { L.Ei += L.U; L.mode = M_STEP; continue; }
         if (L.mode == M_RESTART) { L.mode = M_STEP; continue; }
-        T vc[3];
-        r = second_half<T, GAS>(K, L, vc);
+        r = second_half<T, GAS>(K, L, out);
         if (r == S_CONTINUE) continue;
-        if (r == S_SCATTER) omc = lane_chi<T, GAS>(Kg, L.j, vc[0], vc[1], vc[2]);
+        if (r == S_SCATTER)
+          omc = lane_chi<T, GAS>(Kg, L.j, exit_velocity<T, GAS>(L, 0), exit_velocity<T, GAS>(L, 1),
+                                 exit_velocity<T, GAS>(L, 2));
       }
       // the try has ended: scatter, capped (or watchdog), or a failed test
       if (spec) {
@@ -1948,7 +2136,7 @@ __global__ void __launch_bounds__(BLOCK)
   const size_t grp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
   const size_t ngrp = ((size_t)gridDim.x * blockDim.x) / G;
   for (size_t i = grp; i < npts; i += ngrp) {
-    T p[NS][3], ff[NS][3], UU[NS], cen[3];
+    T p[NS][3], ff[NS][3], row[Row<GAS>::N], cen[3];
     bool act[NS];
     for (int k = 0; k < 3; k++) cen[k] = T(pts[3 * i + k]);
     for (int s = 0; s < NS; s++) {
@@ -1956,11 +2144,13 @@ __global__ void __launch_bounds__(BLOCK)
       act[s] = (s == site) && (kp.allpairs || ref_inside(kp, cen[0], cen[1], cen[2]));
     }
     uint32_t v = 0;
-    eval_forces<T, G, GAS, HASQ>(kp, p, act, cen, T(0), ff, UU, v, g, mask,
-                                 sm_glist + (threadIdx.x & ~(G - 1)) * GCAP_PER_LANE);
+    eval_row<T, G, GAS, HASQ, true>(kp, p, act, cen, T(0), row, v, g, mask,
+                                    sm_glist + (threadIdx.x & ~(G - 1)) * GCAP_PER_LANE);
+    finish_row<T, GAS, HASQ>(kp, row, act, ff);
     if (g == 0) {
       for (int k = 0; k < 3; k++) f[3 * i + k] = (double)ff[site][k];
-      U[i] = (double)UU[site];
+      // one active site: its energy is the probe's
+      U[i] = (double)finish_energy<T, GAS, HASQ>(kp, row, act);
       if (vis) vis[i] = v;
     }
   }

@@ -82,28 +82,14 @@ void vel_table(double m_amu, double T, std::vector<double> &V, std::vector<doubl
   }
 }
 
-template <typename T, int GAS, bool HASQ> KernelFn resume_ptr(int nt) {
-  return nt == 32 ? resume_kernel<T, GAS, HASQ, 32, false>
-                  : nt == 64 ? resume_kernel<T, GAS, HASQ, 64, false> : resume_kernel<T, GAS, HASQ, 128, false>;
-}
 using ForceFn = void (*)(KParams, int, size_t, const double *, double *, double *, uint32_t *);
 
-template <typename T, int G, int GAS, bool HASQ> KernelFn traj_ptr() { return traj_kernel<T, G, GAS, HASQ, false>; }
 template <typename T, int G, int GAS, bool HASQ> ForceFn force_ptr() {
   return force_points_kernel<T, G, GAS, HASQ>;
 }
 
 int g_index(int G) { int i = 0; while ((1 << i) < G) i++; return i; }
 
-template <typename T, int GAS, bool HASQ> KernelFn pick_traj_g(int gi) {
-  switch (gi) {
-    case 0: return traj_ptr<T, 1, GAS, HASQ>();
-    case 2: return traj_ptr<T, 4, GAS, HASQ>();
-    case 3: return traj_ptr<T, 8, GAS, HASQ>();
-    case 4: return traj_ptr<T, 16, GAS, HASQ>();
-    default: return traj_ptr<T, 32, GAS, HASQ>();
-  }
-}
 template <typename T, int GAS, bool HASQ> ForceFn pick_force_g(int gi) {
   switch (gi) {
     case 0: return force_ptr<T, 1, GAS, HASQ>();
@@ -111,21 +97,24 @@ template <typename T, int GAS, bool HASQ> ForceFn pick_force_g(int gi) {
     default: return force_ptr<T, 32, GAS, HASQ>();
   }
 }
-template <typename T> KernelFn pick_traj_t(int gas, bool hasq, int gi) {
-  if (gas == GAS_ATOM) return hasq ? pick_traj_g<T, GAS_ATOM, true>(gi) : pick_traj_g<T, GAS_ATOM, false>(gi);
-  if (gas == GAS_N2) return hasq ? pick_traj_g<T, GAS_N2, true>(gi) : pick_traj_g<T, GAS_N2, false>(gi);
-  return hasq ? pick_traj_g<T, GAS_CO2, true>(gi) : pick_traj_g<T, GAS_CO2, false>(gi);
-}
 template <typename T> ForceFn pick_force_t(int gas, bool hasq, int gi) {
   if (gas == GAS_ATOM) return hasq ? pick_force_g<T, GAS_ATOM, true>(gi) : pick_force_g<T, GAS_ATOM, false>(gi);
   if (gas == GAS_N2) return hasq ? pick_force_g<T, GAS_N2, true>(gi) : pick_force_g<T, GAS_N2, false>(gi);
   return hasq ? pick_force_g<T, GAS_CO2, true>(gi) : pick_force_g<T, GAS_CO2, false>(gi);
 }
+template <typename T> KernelFn pick_lane_t(int gas, bool hasq, int G, bool batch) {
+  return gas == GAS_ATOM ? lane_kernel<T, GAS_ATOM>(hasq, G, batch)
+                         : gas == GAS_N2 ? lane_kernel<T, GAS_N2>(hasq, G, batch) : lane_kernel<T, GAS_CO2>(hasq, G, batch);
+}
+template <typename T> KernelFn pick_warp_t(int gas, bool hasq, int nt, bool batch) {
+  return gas == GAS_ATOM ? warp_kernel<T, GAS_ATOM>(hasq, nt, batch)
+                         : gas == GAS_N2 ? warp_kernel<T, GAS_N2>(hasq, nt, batch) : warp_kernel<T, GAS_CO2>(hasq, nt, batch);
+}
 KernelFn pick_traj(const ccs_ctx *c, int G) {
   const int gas = gas_kind(c->p.gas);
   const bool hasq = c->coul_on || c->dip_on;
-  return c->p.precision == CCS_PREC_FP64 ? pick_traj_t<double>(gas, hasq, g_index(G))
-                                         : pick_traj_t<float>(gas, hasq, g_index(G));
+  return c->p.precision == CCS_PREC_FP64 ? pick_lane_t<double>(gas, hasq, G, false)
+                                         : pick_lane_t<float>(gas, hasq, G, false);
 }
 // threads per trajectory in the warp pass
 // Threads per warp-pass trajectory: the configured value, else 32 for
@@ -143,14 +132,8 @@ KernelFn pick_resume(const ccs_ctx *c) {
   const int gas = gas_kind(c->p.gas);
   const bool hasq = c->coul_on || c->dip_on;
   const int nt = resume_threads(c);
-  if (c->p.precision == CCS_PREC_FP64) {
-    if (gas == GAS_ATOM) return hasq ? resume_ptr<double, GAS_ATOM, true>(nt) : resume_ptr<double, GAS_ATOM, false>(nt);
-    if (gas == GAS_N2) return hasq ? resume_ptr<double, GAS_N2, true>(nt) : resume_ptr<double, GAS_N2, false>(nt);
-    return hasq ? resume_ptr<double, GAS_CO2, true>(nt) : resume_ptr<double, GAS_CO2, false>(nt);
-  }
-  if (gas == GAS_ATOM) return hasq ? resume_ptr<float, GAS_ATOM, true>(nt) : resume_ptr<float, GAS_ATOM, false>(nt);
-  if (gas == GAS_N2) return hasq ? resume_ptr<float, GAS_N2, true>(nt) : resume_ptr<float, GAS_N2, false>(nt);
-  return hasq ? resume_ptr<float, GAS_CO2, true>(nt) : resume_ptr<float, GAS_CO2, false>(nt);
+  return c->p.precision == CCS_PREC_FP64 ? pick_warp_t<double>(gas, hasq, nt, false)
+                                         : pick_warp_t<float>(gas, hasq, nt, false);
 }
 ForceFn pick_force(const ccs_ctx *c, int G) {
   const int gas = gas_kind(c->p.gas);
@@ -231,6 +214,9 @@ KParams ccs_internal::base_params(const ccs_ctx *c) {
   k.work = c->d_work;
   k.stats = c->d_work + 1;
   k.error = c->d_error;
+  k.lane_width = 32;
+  fill_kconst<float>(k);
+  fill_kconst<double>(k);
   return k;
 }
 
@@ -318,6 +304,16 @@ int arm_deadline(ccs_ctx *c, unsigned long long *word, cudaStream_t s) {
   return CCS_OK;
 }
 
+// Grid and trajectories per warp of the lane pass.  A warp evaluates the
+// forces of its probes one after another, so fewer trajectories than lanes
+// in the resident warps are spread over all of them, the fewest per warp.
+void lane_shape(const ccs_ctx *c, size_t n, int per_sm, size_t &grid, int &width) {
+  const size_t warps_cta = BLOCK / 32;
+  grid = (size_t)std::max(per_sm, 1) * c->sm_count;
+  width = (int)std::min<size_t>(32, std::max<size_t>(1, (n + grid * warps_cta - 1) / (grid * warps_cta)));
+  grid = std::min(grid, std::max<size_t>(1, (n + warps_cta * width - 1) / (warps_cta * width)));
+}
+
 // Full asynchronous run on device buffers (no host synchronisation).
 int run_device(ccs_ctx *c, size_t n, const double *d_rnd, size_t stride, int8_t *d_status,
                double *d_omc, uint32_t *d_steps, uint32_t *d_visits, cudaStream_t s, int G,
@@ -339,10 +335,8 @@ int run_device(ccs_ctx *c, size_t n, const double *d_rnd, size_t stride, int8_t 
   if (surr) CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, block, dyn));
-  if (per_sm < 1) per_sm = 1;
-  size_t grid = (size_t)per_sm * c->sm_count;
-  const size_t max_useful = (n + block - 1) / block;  // one trajectory per lane
-  if (grid > max_useful) grid = std::max<size_t>(1, max_useful);
+  size_t grid = 0;
+  lane_shape(c, n, per_sm, grid, k.lane_width);
   k.deadline = c->d_work + 8;
   // longest-expected-first processing order (a radix sort of the length keys)
   if (n > 1 && c->p.schedule == 1) {
@@ -471,25 +465,6 @@ int autotune(ccs_ctx *c, size_t n, size_t stride, int block) {
 // Batched ions: one launch of each pass over the trajectories of many ions.
 // Every ion keeps its own context (parameters, target tables, cell grid); the
 // kernels pick the ion's parameters per trajectory from a device array.
-template <typename T, int G, int GAS, bool HASQ> KernelFn traj_batch_ptr() {
-  return traj_kernel<T, G, GAS, HASQ, true>;
-}
-template <typename T, int GAS, bool HASQ> KernelFn pick_traj_batch_g(int G) {
-  return G <= 8 ? traj_batch_ptr<T, 8, GAS, HASQ>()
-                : G == 16 ? traj_batch_ptr<T, 16, GAS, HASQ>() : traj_batch_ptr<T, 32, GAS, HASQ>();
-}
-template <typename T> KernelFn pick_traj_batch_t(int gas, bool hasq, int G) {
-  if (gas == GAS_ATOM) return hasq ? pick_traj_batch_g<T, GAS_ATOM, true>(G) : pick_traj_batch_g<T, GAS_ATOM, false>(G);
-  if (gas == GAS_N2) return hasq ? pick_traj_batch_g<T, GAS_N2, true>(G) : pick_traj_batch_g<T, GAS_N2, false>(G);
-  return hasq ? pick_traj_batch_g<T, GAS_CO2, true>(G) : pick_traj_batch_g<T, GAS_CO2, false>(G);
-}
-template <typename T> KernelFn pick_resume_batch_t(int gas, bool hasq) {
-  if (gas == GAS_ATOM)
-    return hasq ? resume_kernel<T, GAS_ATOM, true, RBLOCK, true> : resume_kernel<T, GAS_ATOM, false, RBLOCK, true>;
-  if (gas == GAS_N2)
-    return hasq ? resume_kernel<T, GAS_N2, true, RBLOCK, true> : resume_kernel<T, GAS_N2, false, RBLOCK, true>;
-  return hasq ? resume_kernel<T, GAS_CO2, true, RBLOCK, true> : resume_kernel<T, GAS_CO2, false, RBLOCK, true>;
-}
 int batch_lanes(int G) { return G <= 8 ? 8 : G <= 16 ? 16 : 32; }
 
 // Both passes over trajectories [0, m[i]) of every ion i, whose random rows
@@ -568,12 +543,12 @@ int run_batch_device(ccs_ctx *lead, ccs_ctx *const *ions, size_t nions, const si
   const int gas = gas_kind(lead->p.gas);
   const bool fp64 = lead->p.precision == CCS_PREC_FP64;
   const int Gb = batch_lanes(G);
-  KernelFn fn = fp64 ? pick_traj_batch_t<double>(gas, hasq, Gb) : pick_traj_batch_t<float>(gas, hasq, Gb);
-  KernelFn rfn = fp64 ? pick_resume_batch_t<double>(gas, hasq) : pick_resume_batch_t<float>(gas, hasq);
+  KernelFn fn = fp64 ? pick_lane_t<double>(gas, hasq, Gb, true) : pick_lane_t<float>(gas, hasq, Gb, true);
+  KernelFn rfn = fp64 ? pick_warp_t<double>(gas, hasq, RBLOCK, true) : pick_warp_t<float>(gas, hasq, RBLOCK, true);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, BLOCK, 0));
-  size_t grid = (size_t)std::max(per_sm, 1) * lead->sm_count;
-  grid = std::min(grid, std::max<size_t>(1, (total + BLOCK - 1) / BLOCK));
+  size_t grid = 0;
+  lane_shape(lead, total, per_sm, grid, k.lane_width);
   CK(cudaEventRecord(lead->ev[5], s));
   fn<<<(unsigned)grid, BLOCK, 0, s>>>(k, lead->d_kparams);
   CK(cudaGetLastError());
@@ -1286,8 +1261,8 @@ extern "C" int ccs_run_device_noalloc(ccs_ctx *c, size_t n, const double *d_rnd,
   KernelFn fn = pick_traj(c, G);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, block, 0));
-  size_t grid = (size_t)std::max(per_sm, 1) * c->sm_count;
-  grid = std::min(grid, std::max<size_t>(1, (n + block - 1) / block));
+  size_t grid = 0;
+  lane_shape(c, n, per_sm, grid, k.lane_width);
   CK(cudaEventRecord(c->ev[2], s));
   CK(cudaEventRecord(c->ev[5], s));
   fn<<<(unsigned)grid, block, 0, s>>>(k, kparams);

@@ -120,6 +120,21 @@ inline bool is_molecule(int gas) { return gas == CCS_GAS_N2 || gas == CCS_GAS_CO
 inline int gas_kind(int gas) { return gas == CCS_GAS_N2 ? ccs::GAS_N2 : gas == CCS_GAS_CO2 ? ccs::GAS_CO2 : ccs::GAS_ATOM; }
 
 using KernelFn = void (*)(ccs::KParams, const ccs::KParams *);
+// The trajectory kernels of a precision and gas shape (lane_pass.cu and
+// warp_pass.cu, one object each per instantiation): lane pass with G lanes
+// per force evaluation, warp pass with nt threads, single-ion or batched.
+template <typename T, int GAS> KernelFn lane_kernel(bool hasq, int G, bool batch);
+template <typename T, int GAS> KernelFn warp_kernel(bool hasq, int nt, bool batch);
+#define CCS_DECLARE_PASSES(T, GAS)                               \
+  template <> KernelFn lane_kernel<T, GAS>(bool, int, bool);     \
+  template <> KernelFn warp_kernel<T, GAS>(bool, int, bool);
+CCS_DECLARE_PASSES(float, 0)
+CCS_DECLARE_PASSES(float, 1)
+CCS_DECLARE_PASSES(float, 2)
+CCS_DECLARE_PASSES(double, 0)
+CCS_DECLARE_PASSES(double, 1)
+CCS_DECLARE_PASSES(double, 2)
+#undef CCS_DECLARE_PASSES
 // The trajectory kernels with the learned field (traj_field.cu): lane pass
 // with G lanes per exact evaluation, warp pass with nt threads.
 KernelFn pick_traj_field(int gas, bool hasq, int G);
