@@ -52,7 +52,7 @@ ENGINE_UNITS = [("ccs_engine.cu", [], "ccs_engine.o"), ("field.cu", [], "field.o
                 ("traj_field.cu", [], "traj_field.o"), ("setup_gpu.cu", [], "setup_gpu.o")]
 ENGINE_UNITS += [(f"{src}.cu", [f"-DCCS_PASS_T={t}", f"-DCCS_PASS_GAS={g}"], f"{src}_{t}_{g}.o")
                  for src in ("lane_pass", "warp_pass") for t in ("float", "double") for g in (0, 1, 2)]
-ENGINE_HEADERS = ["ccs_device.cuh", "field_device.cuh", "engine_ctx.h"]
+ENGINE_HEADERS = ["ccs_device.cuh", "warp_pass.cuh", "field_device.cuh", "engine_ctx.h"]
 
 
 def build_engine(force=False, verbose=False):

@@ -107,7 +107,8 @@ struct KParams {
   unsigned long long park_cap;
   uint32_t park_steps;
   int park_drained;                 // 1: park only once every trajectory has been taken
-  int lcap;                         // warp pass: candidate-list entries (dynamic shared memory)
+  int lcap;                         // warp pass: most entries of a candidate list
+  int wp_cap, wp_pack;              // warp pass: entries that the shared memory holds; 1: packed candidates too
   // batched ions: per-ion parameters (their rnd/status/omc/steps/visits point
   // at the ion's first trajectory) and the global index of each ion's first
   // trajectory (nions + 1 entries); unused by single-ion runs
@@ -422,7 +423,9 @@ __device__ __forceinline__ bool ref_inside(const KParams &kp, T x, T y, T z) {
 
 // Column (i,j) number cidx of the ncol columns meeting the sphere of radius Rr
 // around c: its z-run of atoms [b, b + len) clipped to the sphere.
-template <typename T>
+// RF: which of the two first products rounds first; it decides borderline
+// cells (one in 1e5 lists), so each kernel keeps one form for good.
+template <bool RF = false, typename T>
 __device__ __forceinline__ void column_run(const KParams &kp, int cidx, int ncol, int i0, int j0, int nj,
                                            float inv_nj, T cx, T cy, T cz, T Rr, int &b, int &len) {
   b = 0;
@@ -435,7 +438,8 @@ __device__ __forceinline__ void column_run(const KParams &kp, int cidx, int ncol
   const T xlo = ox + T(i) * h, ylo = oy + T(j) * h;
   const T dxc = fmax(fmax(xlo - cx, cx - (xlo + h)), T(0));
   const T dyc = fmax(fmax(ylo - cy, cy - (ylo + h)), T(0));
-  const T rem = Rr * Rr - dxc * dxc - dyc * dyc;
+  const T rem = Real<T>::fma(-dyc, dyc, RF ? Real<T>::fma(Rr, Rr, -Real<T>::mul(dxc, dxc))
+                                           : Real<T>::fma(-dxc, dxc, Real<T>::mul(Rr, Rr)));
   if (rem < T(0)) return;
   const T zr = Real<T>::sq(rem);
   const int k0 = (int)fmax(T(0), floor((cz - zr - oz) * ih));
@@ -1284,8 +1288,9 @@ __device__ __noinline__ double lane_chi(const KParams *__restrict__ kpg, unsigne
 }
 
 // First half of a step: kick, drift (constrained for molecules), angle.
+// inv_dt = 1 / L.dt (read for molecules).
 template <typename T, int GAS>
-__device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
+__device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L, T inv_dt) {
   using S = Sites<GAS>;
   const KConst<T> &kc = kconst<T>(kp);
   const T dt = L.dt;
@@ -1319,7 +1324,6 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L) {
     if (det < T(0)) det = T(0);
     const T lam = Real<T>::div(rr - Real<T>::sq(det), r2ij);
     const T cpos = kc.mu12_over_m1 * lam;  // the reference uses mi for both atoms (:1735-1736)
-    const T inv_dt = Real<T>::div(T(1), dt);
     const T ca = cpos * inv_dt, cb = kc.mu12_over_m2 * lam * inv_dt;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -1530,7 +1534,7 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
 
     bool out = false;
     if (L.mode == M_STEP) {
-      first_half<T, GAS>(K, L);
+      first_half<T, GAS>(K, L, GAS == GAS_ATOM ? T(0) : Real<T>::div(T(1), L.dt));
       out = step_leaves(K, L);
     }
 
@@ -1794,6 +1798,91 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
 // the sequential path.
 constexpr int RBLOCK = 64;  // default threads per trajectory in the warp pass
 
+
+// Thread 0's claim of the CTA's next item: a parked trajectory (kind 0), else
+// a speculative try (kind 1); ~0: none is left.
+__device__ __forceinline__ unsigned long long claim_item(const KParams &kp, unsigned long long np,
+                                                         unsigned long long *next, bool spec_launch, bool may_spec,
+                                                         unsigned long long deadline, bool &park_done, int &kind) {
+  unsigned long long v = ~0ull;
+  kind = spec_launch ? 1 : 0;
+  if (*(volatile int *)kp.error) return v;
+  if (!park_done) {
+    if (may_spec) atomicAdd(kp.park_active, 1ull);  // before taking: a poller never misses it
+    v = atomicAdd(next, 1ull);
+    if (v >= np) {
+      v = ~0ull;
+      park_done = true;
+      if (may_spec) atomicAdd(kp.park_active, ~0ull);  // minus one
+    }
+  } else if (spec_launch) {
+    v = atomicAdd(next, 1ull);
+    if (v >= np) v = ~0ull;
+  }
+  if (v == ~0ull && may_spec) {
+    kind = 1;
+    for (unsigned poll = 0; poll < (1u << 26); poll++) {
+      if ((poll & 255u) == 255u && (global_ns() > deadline || *(volatile int *)kp.error)) {
+        atomicExch(kp.error, 1);  // the watchdog: stop waiting
+        break;
+      }
+      // the running count first: once it is zero every record is published
+      const unsigned long long active = *(volatile unsigned long long *)kp.park_active;
+      __threadfence();
+      unsigned long long cnt = *(volatile unsigned long long *)kp.spec_count;
+      if (cnt > kp.spec_cap) cnt = kp.spec_cap;
+      const unsigned long long cur = *(volatile unsigned long long *)kp.spec_next;
+      if (cur < cnt * SPEC_SLOTS) {
+        if (*(volatile int *)&kp.spec_rec[cur / SPEC_SLOTS].ready &&
+            atomicCAS(kp.spec_next, cur, cur + 1) == cur) {
+          v = cur;
+          break;
+        }
+        continue;  // being published, or another CTA took it: look again
+      }
+      if (active == 0) break;  // nothing left to come
+      __nanosleep(2000);
+    }
+    __threadfence();  // the record's fields after its ready flag
+  }
+  return v;
+}
+
+// The outcome of a speculative try (L.tries of record rec).
+template <typename T>
+__device__ __forceinline__ void write_spec_out(const KParams &kp, unsigned long long rec, const LaneState<T> &L, int r,
+                                               double omc) {
+  SpecOut o;
+  o.omc = omc;
+  o.steps = L.nsteps;
+  o.nvis = L.nvis;
+  o.code = r == S_SCATTER ? 1 : r == S_CAPPED ? 3 : r == S_RETRY_ANGLE ? 4 : 5;
+  o.pad = 0;
+  kp.spec_out[rec * SPEC_SLOTS + (L.tries - __ldcg(&kp.spec_rec[rec].tries))] = o;
+}
+
+// Hands a trajectory's remaining tries over, if the pass is short of work and
+// the records have room; thread 0 only.
+template <typename T>
+__device__ __forceinline__ bool record_spec(const KParams &kp, unsigned long long np, const LaneState<T> &L) {
+  const bool drained = np <= kp.spec_max_parked || *(volatile unsigned long long *)kp.park_next >= np;
+  const unsigned long long slot = drained ? atomicAdd(kp.spec_count, 1ull) : ~0ull;
+  if (slot >= kp.spec_cap) return false;
+  SpecRec R;
+  R.Ei = (double)L.Ei;
+  R.j = L.j;
+  R.ion = L.ion;
+  R.nsteps = L.nsteps;
+  R.nvis = L.nvis;
+  R.tries = L.tries;
+  R.maxTries = L.maxTries;
+  R.ready = 0;
+  kp.spec_rec[slot] = R;
+  __threadfence();  // the fields before the flag that publishes them
+  *(volatile int *)&kp.spec_rec[slot].ready = 1;
+  return true;
+}
+
 // SURR: steps whose sites all lie outside the learned field's exact zone are
 // evaluated by the field, one warp per site (field_site_warp).
 template <typename T, int GAS, bool HASQ, int NT, bool BATCH, bool SURR = false>
@@ -1837,49 +1926,8 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
   __shared__ int sm_kind;
   for (;;) {
     if (tid == 0) {
-      unsigned long long v = ~0ull;
-      int kind = spec_launch ? 1 : 0;
-      if (!*(volatile int *)kp.error) {
-        if (!park_done) {
-          if (may_spec) atomicAdd(kp.park_active, 1ull);  // before taking: a poller never misses it
-          v = atomicAdd(next, 1ull);
-          if (v >= np) {
-            v = ~0ull;
-            park_done = true;
-            if (may_spec) atomicAdd(kp.park_active, ~0ull);  // minus one
-          }
-        } else if (spec_launch) {
-          v = atomicAdd(next, 1ull);
-          if (v >= np) v = ~0ull;
-        }
-        if (v == ~0ull && may_spec) {
-          kind = 1;
-          for (unsigned poll = 0; poll < (1u << 26); poll++) {
-            if ((poll & 255u) == 255u && (global_ns() > deadline || *(volatile int *)kp.error)) {
-              atomicExch(kp.error, 1);  // the watchdog: stop waiting
-              break;
-            }
-            // the running count first: once it is zero every record is published
-            const unsigned long long active = *(volatile unsigned long long *)kp.park_active;
-            __threadfence();
-            unsigned long long cnt = *(volatile unsigned long long *)kp.spec_count;
-            if (cnt > kp.spec_cap) cnt = kp.spec_cap;
-            const unsigned long long cur = *(volatile unsigned long long *)kp.spec_next;
-            if (cur < cnt * SPEC_SLOTS) {
-              if (*(volatile int *)&kp.spec_rec[cur / SPEC_SLOTS].ready &&
-                  atomicCAS(kp.spec_next, cur, cur + 1) == cur) {
-                v = cur;
-                break;
-              }
-              continue;  // being published, or another CTA took it: look again
-            }
-            if (active == 0) break;  // nothing left to come
-            __nanosleep(2000);
-          }
-          __threadfence();  // the record's fields after its ready flag
-        }
-      }
-      sm_idx = v;
+      int kind;
+      sm_idx = claim_item(kp, np, next, spec_launch, may_spec, deadline, park_done, kind);
       sm_kind = kind;
     }
     __syncthreads();
@@ -1932,7 +1980,7 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
       if (r == S_CONTINUE) {
         bool out = false;
         if (L.mode == M_STEP) {
-          first_half<T, GAS>(K, L);
+          first_half<T, GAS>(K, L, GAS == GAS_ATOM ? T(0) : Real<T>::div(T(1), L.dt));
           out = step_leaves(K, L);
         }
         T p[NS][3], fs[NS][3];
@@ -2013,15 +2061,7 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
       }
       // the try has ended: scatter, capped (or watchdog), or a failed test
       if (spec) {
-        if (tid == 0) {
-          SpecOut o;
-          o.omc = omc;
-          o.steps = L.nsteps;
-          o.nvis = L.nvis;
-          o.code = r == S_SCATTER ? 1 : r == S_CAPPED ? 3 : r == S_RETRY_ANGLE ? 4 : 5;
-          o.pad = 0;
-          kp.spec_out[rec * SPEC_SLOTS + (L.tries - __ldcg(&kp.spec_rec[rec].tries))] = o;
-        }
+        if (tid == 0) write_spec_out(kp, rec, L, r, omc);
         break;
       }
       if (r == S_SCATTER) {
@@ -2040,27 +2080,9 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
         break;
       }
       if (may_spec && !spec && L.tries >= kp.spec_from) {  // hand the remaining tries to the speculative phase
-        if (tid == 0) {
-          const bool drained = np <= kp.spec_max_parked || *(volatile unsigned long long *)kp.park_next >= np;
-          const unsigned long long slot = drained ? atomicAdd(kp.spec_count, 1ull) : ~0ull;
-          sm_idx = slot;
-          if (slot < kp.spec_cap) {
-            SpecRec R;
-            R.Ei = (double)L.Ei;
-            R.j = L.j;
-            R.ion = L.ion;
-            R.nsteps = L.nsteps;
-            R.nvis = L.nvis;
-            R.tries = L.tries;
-            R.maxTries = L.maxTries;
-            R.ready = 0;
-            kp.spec_rec[slot] = R;
-            __threadfence();  // the fields before the flag that publishes them
-            *(volatile int *)&kp.spec_rec[slot].ready = 1;
-          }
-        }
+        if (tid == 0) sm_idx = record_spec(kp, np, L) ? 1ull : 0ull;
         __syncthreads();
-        const bool recorded = sm_idx < kp.spec_cap;
+        const bool recorded = sm_idx != 0;
         __syncthreads();
         if (recorded) break;
       }

@@ -106,7 +106,7 @@ template <typename T> KernelFn pick_lane_t(int gas, bool hasq, int G, bool batch
   return gas == GAS_ATOM ? lane_kernel<T, GAS_ATOM>(hasq, G, batch)
                          : gas == GAS_N2 ? lane_kernel<T, GAS_N2>(hasq, G, batch) : lane_kernel<T, GAS_CO2>(hasq, G, batch);
 }
-template <typename T> KernelFn pick_warp_t(int gas, bool hasq, int nt, bool batch) {
+template <typename T> WarpKernel pick_warp_t(int gas, bool hasq, int nt, bool batch) {
   return gas == GAS_ATOM ? warp_kernel<T, GAS_ATOM>(hasq, nt, batch)
                          : gas == GAS_N2 ? warp_kernel<T, GAS_N2>(hasq, nt, batch) : warp_kernel<T, GAS_CO2>(hasq, nt, batch);
 }
@@ -128,7 +128,7 @@ int resume_threads(const ccs_ctx *c) {
   return RBLOCK;
 }
 
-KernelFn pick_resume(const ccs_ctx *c) {
+WarpKernel pick_resume(const ccs_ctx *c) {
   const int gas = gas_kind(c->p.gas);
   const bool hasq = c->coul_on || c->dip_on;
   const int nt = resume_threads(c);
@@ -255,21 +255,45 @@ int setup_spec(ccs_ctx *c, KParams &k, size_t cap, cudaStream_t s) {
   return CCS_OK;
 }
 
+// Grid and shared memory of a warp-pass kernel, with the sizes that the
+// kernel reads (k.lcap set): the candidate list, its packed copy where that
+// leaves room for four CTAs on an SM (FP32, lists of up to about 2000
+// candidates: a step then reads 24 B in list order instead of an index and a
+// gather), and with the learned field the near-part list.
+int warp_shape(ccs_ctx *c, const WarpKernel &wk, KParams &k, size_t most_atoms, size_t &grid, size_t &dyn) {
+  k.wp_cap = (int)((std::min<size_t>(k.lcap, most_atoms) + 3) / 4 * 4);
+  k.wp_pack = 0;
+  dyn = (size_t)(k.lcap + LCAP) * sizeof(int);
+  if (!k.field.on) {
+    dyn = (size_t)k.wp_cap * sizeof(int);
+    const size_t packed = (size_t)k.wp_cap * (sizeof(float4) + (c->p.gas == CCS_GAS_CO2 ? 2 : 1) * sizeof(float2));
+    if (c->p.precision != CCS_PREC_FP64 && dyn + packed <= 58 * 1024) {
+      k.wp_pack = 1;
+      dyn += packed;
+    }
+  }
+  if (dyn > 32 * 1024)
+    CK(cudaFuncSetAttribute((const void *)wk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)wk.fn, wk.threads, dyn));
+  grid = (size_t)std::max(per_sm, 1) * c->sm_count;
+  return CCS_OK;
+}
+
 // The warp pass: parked trajectories (phase 0), the speculative tries of
 // those that failed spec_from tries there (phase 1), their verdicts.
 template <bool BATCH>
-int launch_warp_pass(ccs_ctx *c, KernelFn rfn, int rnt, KParams k, cudaStream_t s) {
-  int rper_sm = 0;
-  // the candidate list (and with the learned field the near-part list)
-  const size_t dyn = (size_t)(k.lcap + (k.field.on ? LCAP : 0)) * sizeof(int);
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rper_sm, (const void *)rfn, rnt, dyn));
-  const unsigned rgrid = (unsigned)((size_t)std::max(rper_sm, 1) * c->sm_count);
+int launch_warp_pass(ccs_ctx *c, const WarpKernel &wk, KParams k, size_t most_atoms, cudaStream_t s) {
+  size_t grid = 0, dyn = 0;
+  int rc = warp_shape(c, wk, k, most_atoms, grid, dyn);
+  if (rc) return rc;
+  const unsigned rgrid = (unsigned)grid;
   k.spec_max_parked = 2ull * rgrid;  // measured: 448 parked of 3e5 (60 atoms, He) 1.7x faster, 52,241 (1231 atoms, N2) slower
-  rfn<<<rgrid, rnt, dyn, s>>>(k, c->d_kparams);
+  wk.fn<<<rgrid, wk.threads, dyn, s>>>(k, c->d_kparams);
   CK(cudaGetLastError());
   if (k.spec_rec) {
     k.spec_phase = 1;
-    rfn<<<rgrid, rnt, dyn, s>>>(k, c->d_kparams);
+    wk.fn<<<rgrid, wk.threads, dyn, s>>>(k, c->d_kparams);
     CK(cudaGetLastError());
     spec_resolve_kernel<BATCH><<<(unsigned)((k.spec_cap + 255) / 256), 256, 0, s>>>(k);
     CK(cudaGetLastError());
@@ -396,8 +420,9 @@ int run_device(ccs_ctx *c, size_t n, const double *d_rnd, size_t stride, int8_t 
   CK(cudaGetLastError());
   CK(cudaEventRecord(c->ev[6], s));
   // warp pass over the parked trajectories (exits at once when none were parked)
-  KernelFn rfn = surr ? pick_resume_field(gas_kind(c->p.gas), hasq, resume_threads(c)) : pick_resume(c);
-  rc = launch_warp_pass<false>(c, rfn, resume_threads(c), k, s);
+  const int rnt = resume_threads(c);
+  const WarpKernel wk = surr ? WarpKernel{pick_resume_field(gas_kind(c->p.gas), hasq, rnt), rnt} : pick_resume(c);
+  rc = launch_warp_pass<false>(c, wk, k, c->natoms, s);
   if (rc) return rc;
   CK(cudaEventRecord(c->ev[7], s));
   c->last.grid_size = (int32_t)grid;
@@ -544,7 +569,7 @@ int run_batch_device(ccs_ctx *lead, ccs_ctx *const *ions, size_t nions, const si
   const bool fp64 = lead->p.precision == CCS_PREC_FP64;
   const int Gb = batch_lanes(G);
   KernelFn fn = fp64 ? pick_lane_t<double>(gas, hasq, Gb, true) : pick_lane_t<float>(gas, hasq, Gb, true);
-  KernelFn rfn = fp64 ? pick_warp_t<double>(gas, hasq, RBLOCK, true) : pick_warp_t<float>(gas, hasq, RBLOCK, true);
+  const WarpKernel wk = fp64 ? pick_warp_t<double>(gas, hasq, RBLOCK, true) : pick_warp_t<float>(gas, hasq, RBLOCK, true);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, BLOCK, 0));
   size_t grid = 0;
@@ -553,7 +578,9 @@ int run_batch_device(ccs_ctx *lead, ccs_ctx *const *ions, size_t nions, const si
   fn<<<(unsigned)grid, BLOCK, 0, s>>>(k, lead->d_kparams);
   CK(cudaGetLastError());
   CK(cudaEventRecord(lead->ev[6], s));
-  rc = launch_warp_pass<true>(lead, rfn, RBLOCK, k, s);
+  size_t most_atoms = 0;
+  for (size_t i = 0; i < nions; i++) most_atoms = std::max<size_t>(most_atoms, ions[i]->natoms);
+  rc = launch_warp_pass<true>(lead, wk, k, most_atoms, s);
   if (rc) return rc;
   CK(cudaEventRecord(lead->ev[7], s));
   lead->last.grid_size = (int32_t)grid;
@@ -1268,12 +1295,11 @@ extern "C" int ccs_run_device_noalloc(ccs_ctx *c, size_t n, const double *d_rnd,
   fn<<<(unsigned)grid, block, 0, s>>>(k, kparams);
   CK(cudaGetLastError());
   CK(cudaEventRecord(c->ev[6], s));
-  KernelFn rfn = pick_resume(c);
-  int rper_sm = 0;
-  const int rnt = resume_threads(c);
-  const size_t rdyn = (size_t)k.lcap * sizeof(int);
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rper_sm, (const void *)rfn, rnt, rdyn));
-  rfn<<<(unsigned)((size_t)std::max(rper_sm, 1) * c->sm_count), rnt, rdyn, s>>>(k, kparams);
+  const WarpKernel wk = pick_resume(c);
+  size_t rgrid = 0, rdyn = 0;
+  rc = warp_shape(c, wk, k, c->natoms, rgrid, rdyn);
+  if (rc) return rc;
+  wk.fn<<<(unsigned)rgrid, wk.threads, rdyn, s>>>(k, kparams);
   CK(cudaGetLastError());
   CK(cudaEventRecord(c->ev[7], s));
   CK(cudaEventRecord(c->ev[3], s));

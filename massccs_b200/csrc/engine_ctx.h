@@ -122,12 +122,17 @@ inline int gas_kind(int gas) { return gas == CCS_GAS_N2 ? ccs::GAS_N2 : gas == C
 using KernelFn = void (*)(ccs::KParams, const ccs::KParams *);
 // The trajectory kernels of a precision and gas shape (lane_pass.cu and
 // warp_pass.cu, one object each per instantiation): lane pass with G lanes
-// per force evaluation, warp pass with nt threads, single-ion or batched.
+// per force evaluation, warp pass with nt virtual threads per trajectory
+// (`threads` in the CTA: one warp per role), single-ion or batched.
+struct WarpKernel {
+  KernelFn fn;
+  int threads;
+};
 template <typename T, int GAS> KernelFn lane_kernel(bool hasq, int G, bool batch);
-template <typename T, int GAS> KernelFn warp_kernel(bool hasq, int nt, bool batch);
+template <typename T, int GAS> WarpKernel warp_kernel(bool hasq, int nt, bool batch);
 #define CCS_DECLARE_PASSES(T, GAS)                               \
   template <> KernelFn lane_kernel<T, GAS>(bool, int, bool);     \
-  template <> KernelFn warp_kernel<T, GAS>(bool, int, bool);
+  template <> WarpKernel warp_kernel<T, GAS>(bool, int, bool);
 CCS_DECLARE_PASSES(float, 0)
 CCS_DECLARE_PASSES(float, 1)
 CCS_DECLARE_PASSES(float, 2)

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) far_label_kernel(KParams kp, FieldKind fk
     const int ncol = column_range<float>(kp, P.x, P.y, R, i0, j0, nj, inv_nj);
     for (int c = lane; c < ncol; c += 32) {
       int b, len;
-      column_run<float>(kp, c, ncol, i0, j0, nj, inv_nj, P.x, P.y, P.z, R, b, len);
+      column_run(kp, c, ncol, i0, j0, nj, inv_nj, P.x, P.y, P.z, R, b, len);
       for (int ai = b; ai < b + len; ai++) {
         const float4 a = __ldg(&kp.xyzq32[ai]);
         const float dx = P.x - a.x, dy = P.y - a.y, dz = P.z - a.z;
