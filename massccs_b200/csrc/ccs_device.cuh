@@ -573,6 +573,9 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
   for (int s = 0; s < NS; s++) any |= act[s];
   if (!any) return;
   uint32_t nvis = 0;
+  // candidates in flight at once: their loads, rsqrt and products overlap,
+  // their sums keep the list's order
+  constexpr int U = G == 1 ? 1 : NS == 1 ? 4 : 2;
   const KConst<T> &kc = kconst<T>(kp);
   // candidate sphere around the centre; +1e-3 A so rounding never drops a pair
   // (the near part of the range separation reaches r_out only)
@@ -587,10 +590,17 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
   if ((G > 1 && kp.natoms <= 2 * G) || fx * fx + fy * fy + fz * fz <= R * R) {
     // the whole target inside the reach sphere, or a target of at most two
     // atoms per lane of the group: every atom is a candidate
-    for (int ai = g; ai < kp.natoms; ai += G) {
-      const Atom<T> a = load_atom<T, GAS>(kp, ai);
-      visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a, acc);
+    int ai = g;
+    for (; ai + (U - 1) * G < kp.natoms; ai += U * G) {
+      Atom<T> a[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) a[u] = load_atom<T, GAS>(kp, ai + u * G);
+#pragma unroll
+      for (int u = 0; u < U; u++) visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a[u], acc);
     }
+    if constexpr (U > 1)
+      for (; ai < kp.natoms; ai += G)
+        visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, load_atom<T, GAS>(kp, ai), acc);
     if (G == 1 || g == 0) nvis += (uint32_t)kp.natoms;
   } else if (ex * ex + ey * ey + ez * ez <= R * R) {
     int i0, j0, nj;
@@ -615,6 +625,39 @@ __device__ __forceinline__ void accumulate_group(const KParams &kp, const T (&p)
         }
         const int total = __shfl_sync(mask, incl, G - 1, G);
         const int excl = incl - len;
+        if constexpr (G == 32) {
+          // Candidate t of the batch lies in the last run that starts at or
+          // before t.  Each 32 candidates' starts are one word, so a lane's run
+          // is a population count away; writing the runs out to a list instead
+          // took a loop over the longest run (up to 80 atoms) of one lane each.
+          const unsigned le = 0xffffffffu >> (31 - g);
+          const unsigned filled = __ballot_sync(mask, len > 0);
+          if (len > 0) glist[__popc(filled & (le >> 1))] = b - excl;  // run number -> atom minus candidate
+          __syncwarp(mask);
+          const int word = len > 0 ? excl >> 5 : -1;
+          const unsigned bit = 1u << (excl & 31);
+          int runs = -1;  // runs that start before the 32 at hand, less one
+          auto atom_of = [&](int t0) {
+            const unsigned starts = __reduce_or_sync(mask, word == (t0 >> 5) ? bit : 0u);
+            const int run = runs + __popc(starts & le);
+            runs += __popc(starts);
+            return t0 + g + glist[run];
+          };
+          int t0 = 0;
+          for (; t0 + 32 * U <= total; t0 += 32 * U) {
+            Atom<T> a[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) a[u] = load_atom<T, GAS>(kp, atom_of(t0 + 32 * u));
+#pragma unroll
+            for (int u = 0; u < U; u++) visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, a[u], acc);
+          }
+          for (; t0 < total; t0 += 32) {
+            const int ai = atom_of(t0);
+            if (t0 + g < total)
+              visit_atom<T, GAS, HASQ, SPLIT, WF, WU, sizeof(T) == 8>(kp, p, act, load_atom<T, GAS>(kp, ai), acc);
+          }
+          __syncwarp(mask);  // the runs are rewritten next
+        } else
         for (int cs = 0; cs < total; cs += GCAP) {
           const int lo = max(excl, cs), hi = min(excl + len, cs + GCAP);
           for (int q = lo; q < hi; q++) glist[q - cs] = b + (q - excl);
