@@ -179,14 +179,16 @@ static __global__ void arm_watchdog(unsigned long long *deadline, unsigned long 
   *deadline = global_ns() + budget_ns;
 }
 
-// A trajectory handed to the speculative phase: it failed try tries - 1 and
-// will run tries tries..8 (the reference never runs a tenth: tries < maxTries
-// <= 9), all at once, one CTA each.
+// A trajectory whose tries run at once: it failed try tries - 1 and will run
+// tries tries..8 (the reference never runs a tenth: tries < maxTries <= 9),
+// one CTA each, the first in the CTA that had the trajectory.
 struct SpecRec {
   double Ei;                  // initial total energy (the same for every try)
   unsigned long long j;
   uint32_t ion, nsteps, nvis; // steps and visits of the tries before
   int tries, maxTries;
+  int stop;                   // the decision falls at this try or before: later ones need not run
+  unsigned ended, energy;     // tries that ended without a verdict, by either test, and by the energy test
   int ready;                  // set (after a fence) once the fields above are written
 };
 
@@ -201,6 +203,8 @@ __device__ __forceinline__ SpecRec load_spec_rec(const SpecRec *p) {
   R.nvis = __ldcg(&p->nvis);
   R.tries = __ldcg(&p->tries);
   R.maxTries = __ldcg(&p->maxTries);
+  R.stop = *(const volatile int *)&p->stop;
+  R.ended = R.energy = 0;
   R.ready = 1;
   return R;
 }
@@ -211,8 +215,9 @@ struct SpecOut {
   uint32_t steps, nvis;
   int code, pad;
 };
-constexpr int SPEC_FROM_MIN = 2;  // the fewest failed tries after which speculation starts
-constexpr int SPEC_SLOTS = 9 - SPEC_FROM_MIN;  // tries tries..tries+6 (those above 8 are skipped)
+constexpr int SPEC_FROM_MIN = 1;  // the fewest failed tries after which speculation starts
+constexpr int SPEC_SLOTS = 9 - SPEC_FROM_MIN;  // tries tries..tries+7 (those above 8 are skipped)
+constexpr int SPEC_ITEMS = SPEC_SLOTS - 1;     // of these, the ones that other CTAs take
 
 template <typename T> struct Real;
 // fma/mul/add: single roundings that the compiler neither fuses nor splits,
@@ -1875,8 +1880,8 @@ __device__ __forceinline__ unsigned long long claim_item(const KParams &kp, unsi
       unsigned long long cnt = *(volatile unsigned long long *)kp.spec_count;
       if (cnt > kp.spec_cap) cnt = kp.spec_cap;
       const unsigned long long cur = *(volatile unsigned long long *)kp.spec_next;
-      if (cur < cnt * SPEC_SLOTS) {
-        if (*(volatile int *)&kp.spec_rec[cur / SPEC_SLOTS].ready &&
+      if (cur < cnt * SPEC_ITEMS) {
+        if (*(volatile int *)&kp.spec_rec[cur / SPEC_ITEMS].ready &&
             atomicCAS(kp.spec_next, cur, cur + 1) == cur) {
           v = cur;
           break;
@@ -1891,26 +1896,52 @@ __device__ __forceinline__ unsigned long long claim_item(const KParams &kp, unsi
   return v;
 }
 
-// The outcome of a speculative try (L.tries of record rec).
+// The outcome of a speculative try (L.tries of record rec), and the tries
+// that it makes needless: those after one that scatters or is capped; after
+// the energy failure that reaches the limit (each grants a try, and the tenth
+// granted try ends the trajectory); and try 8 once all before it have failed
+// the angle test.
 template <typename T>
 __device__ __forceinline__ void write_spec_out(const KParams &kp, unsigned long long rec, const LaneState<T> &L, int r,
                                                double omc) {
+  SpecRec *const R = kp.spec_rec + rec;
+  const int first = __ldcg(&R->tries), most = __ldcg(&R->maxTries);
+  if (r == S_SCATTER || r == S_CAPPED) {
+    atomicMin(&R->stop, L.tries);
+  } else {
+    // a try's energy bit is set before its ended bit, and read after it: whoever
+    // sees every try ended sees every energy failure
+    if (r == S_RETRY_ENERGY) atomicOr(&R->energy, 1u << L.tries);
+    __threadfence();
+    const unsigned ended = atomicOr(&R->ended, 1u << L.tries) | 1u << L.tries;
+    __threadfence();
+    const unsigned energy = atomicOr(&R->energy, 0u);
+    const unsigned before8 = 0xffu & ~((1u << first) - 1u);
+    if (energy == 0 && most == 8 && (ended & before8) == before8) atomicMin(&R->stop, 7);
+    int left = 10 - most;
+    for (int k = first; k <= 8; k++)
+      if ((energy >> k & 1u) && --left <= 0) {
+        atomicMin(&R->stop, k);
+        break;
+      }
+  }
   SpecOut o;
   o.omc = omc;
   o.steps = L.nsteps;
   o.nvis = L.nvis;
   o.code = r == S_SCATTER ? 1 : r == S_CAPPED ? 3 : r == S_RETRY_ANGLE ? 4 : 5;
   o.pad = 0;
-  kp.spec_out[rec * SPEC_SLOTS + (L.tries - __ldcg(&kp.spec_rec[rec].tries))] = o;
+  kp.spec_out[rec * SPEC_SLOTS + (L.tries - first)] = o;
 }
 
-// Hands a trajectory's remaining tries over, if the pass is short of work and
-// the records have room; thread 0 only.
+// Records a trajectory for its remaining tries (L.tries goes on in the
+// caller's CTA), if the pass is short of work and the records have room;
+// thread 0 only.  Returns the record, or ~0.
 template <typename T>
-__device__ __forceinline__ bool record_spec(const KParams &kp, unsigned long long np, const LaneState<T> &L) {
+__device__ __forceinline__ unsigned long long record_spec(const KParams &kp, unsigned long long np, const LaneState<T> &L) {
   const bool drained = np <= kp.spec_max_parked || *(volatile unsigned long long *)kp.park_next >= np;
   const unsigned long long slot = drained ? atomicAdd(kp.spec_count, 1ull) : ~0ull;
-  if (slot >= kp.spec_cap) return false;
+  if (slot >= kp.spec_cap) return ~0ull;
   SpecRec R;
   R.Ei = (double)L.Ei;
   R.j = L.j;
@@ -1919,11 +1950,15 @@ __device__ __forceinline__ bool record_spec(const KParams &kp, unsigned long lon
   R.nvis = L.nvis;
   R.tries = L.tries;
   R.maxTries = L.maxTries;
+  R.stop = 9;
+  R.ended = R.energy = 0;
   R.ready = 0;
   kp.spec_rec[slot] = R;
   __threadfence();  // the fields before the flag that publishes them
   *(volatile int *)&kp.spec_rec[slot].ready = 1;
-  return true;
+  __threadfence();
+  atomicAdd(kp.park_active, ~0ull);  // its tries are records now: one fewer parked trajectory running
+  return slot;
 }
 
 // SURR: steps whose sites all lie outside the learned field's exact zone are
@@ -1949,7 +1984,7 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
   if (spec_launch) {
     np = *(volatile unsigned long long *)kp.spec_count;
     if (np > kp.spec_cap) np = kp.spec_cap;
-    np *= SPEC_SLOTS;
+    np *= SPEC_ITEMS;
   } else {
     np = *(volatile unsigned long long *)kp.park_count;
     if (np > kp.park_cap) np = kp.park_cap;
@@ -1975,15 +2010,15 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
     }
     __syncthreads();
     const unsigned long long idx = sm_idx;
-    const bool spec = sm_kind != 0;  // this item is a speculative try
+    bool spec = sm_kind != 0;  // this item is a speculative try
     __syncthreads();
     if (idx == ~0ull) break;
     LaneState<T> L;
     unsigned long long rec = 0;
     if (spec) {  // try k of record rec, from the trajectory's initial state
-      rec = idx / SPEC_SLOTS;
+      rec = idx / SPEC_ITEMS;
       const SpecRec R = load_spec_rec(kp.spec_rec + rec);
-      const int k = R.tries + (int)(idx % SPEC_SLOTS);
+      const int k = R.tries + 1 + (int)(idx % SPEC_ITEMS);
       if (k > 8) continue;  // beyond the reference's last try (block-uniform)
       L.j = R.j;
       L.ion = R.ion;
@@ -2122,12 +2157,16 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
         if (tid == 0) write_result(K, L, 2, 0.0, blk);
         break;
       }
-      if (may_spec && !spec && L.tries >= kp.spec_from) {  // hand the remaining tries to the speculative phase
-        if (tid == 0) sm_idx = record_spec(kp, np, L) ? 1ull : 0ull;
+      if (may_spec && L.tries >= kp.spec_from) {  // the remaining tries at once, this one here
+        if (tid == 0) sm_idx = record_spec(kp, np, L);
         __syncthreads();
-        const bool recorded = sm_idx != 0;
+        const unsigned long long slot = sm_idx;
         __syncthreads();
-        if (recorded) break;
+        if (slot != ~0ull) {
+          spec = true;
+          rec = slot;
+          L.nsteps = L.nvis = 0;  // the record holds those so far
+        }
       }
       load_init<T, GAS>(L, lane_setup<T, GAS>(Kg, L.j));
       L.mode = M_RESTART;

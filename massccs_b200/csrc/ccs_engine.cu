@@ -247,7 +247,7 @@ int setup_spec(ccs_ctx *c, KParams &k, size_t cap, cudaStream_t s) {
   k.park_active = c->d_work + 13;
   k.spec_cap = cap;
   k.spec_phase = 0;
-  k.spec_from = std::max(SPEC_FROM_MIN, c->p.spec_tries > 0 ? c->p.spec_tries : 2);
+  k.spec_from = std::max(SPEC_FROM_MIN, c->p.spec_tries > 0 ? c->p.spec_tries : 1);
   if (c->p.spec_tries < 0) k.spec_rec = nullptr;  // speculation off
   CK(cudaMemsetAsync(c->d_work + 11, 0, 3 * sizeof(unsigned long long), s));
   // every record unpublished (phase-0 CTAs claim only published records' tries)

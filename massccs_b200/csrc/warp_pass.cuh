@@ -219,7 +219,7 @@ template <typename T, int GAS, int NT> struct WarpShared {
   int wsum[NW];
   unsigned long long blk[8];
   unsigned long long idx;
-  int kind;
+  int kind, stop;
 };
 
 // Exclusive scan of the run lengths of the NT threads of role 0 (every thread
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
   if (spec_launch) {
     np = *(volatile unsigned long long *)kp.spec_count;
     if (np > kp.spec_cap) np = kp.spec_cap;
-    np *= SPEC_SLOTS;
+    np *= SPEC_ITEMS;
   } else {
     np = *(volatile unsigned long long *)kp.park_count;
     if (np > kp.park_cap) np = kp.park_cap;
@@ -356,16 +356,20 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
     }
     __syncthreads();
     const unsigned long long idx = sm.idx;
-    const bool spec = sm.kind != 0;  // this item is a speculative try
+    bool spec = sm.kind != 0;  // this item is a speculative try
     __syncthreads();
     if (idx == ~0ull) break;
     LaneState<T> L;
     unsigned long long rec = 0;
     if (spec) {  // try k of record rec, from the trajectory's initial state
-      rec = idx / SPEC_SLOTS;
+      rec = idx / SPEC_ITEMS;
+      if (tid == 0) sm.stop = *(volatile int *)&kp.spec_rec[rec].stop;
+      __syncthreads();
+      const int stop = sm.stop;
+      __syncthreads();
       const SpecRec R = load_spec_rec(kp.spec_rec + rec);
-      const int k = R.tries + (int)(idx % SPEC_SLOTS);
-      if (k > 8) continue;  // beyond the reference's last try (block-uniform)
+      const int k = R.tries + 1 + (int)(idx % SPEC_ITEMS);
+      if (k > 8 || k > stop) continue;  // beyond the last try, or decided before it (block-uniform)
       L.j = R.j;
       L.ion = R.ion;
       load_init<T, GAS>(L, lane_setup<T, GAS>(ion_params_ptr<BATCH>(kp, kpg, L.ion), L.j));
@@ -400,17 +404,38 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
     int list_n = -1;  // this trajectory's candidate list (none yet)
     T list_c[3] = {T(0), T(0), T(0)};
     T inv_dt = Real<T>::div(T(1), L.dt);
+    // From spec_from failed tries on, the remaining ones run at once as soon
+    // as the pass is short of work; the one at hand goes on here.
+    auto try_record = [&]() {
+      if (tid == 0) sm.idx = record_spec(kp, np, L);
+      __syncthreads();
+      const unsigned long long slot = sm.idx;
+      __syncthreads();
+      if (slot != ~0ull) {
+        spec = true;
+        rec = slot;
+        L.nsteps = L.nvis = 0;  // the record holds those so far
+      }
+    };
+    if (may_spec && !spec && L.tries >= kp.spec_from) try_record();
     for (unsigned it = 1;; it++) {
       int r = S_CONTINUE;
       double omc = 0.0;
-      if ((it & 1023u) == 0) {
-        if (tid == 0) sm.idx = (global_ns() > deadline || *(volatile int *)kp.error) ? 1ull : 0ull;
+      if ((it & 255u) == 0) {
+        if (tid == 0) {
+          sm.stop = (global_ns() > deadline || *(volatile int *)kp.error)                   ? 1
+                    : spec && L.tries > *(volatile int *)&kp.spec_rec[rec].stop ? 2
+                                                                                : 0;
+        }
         __syncthreads();
-        const bool e = sm.idx != 0;
+        const int e = sm.stop;
         __syncthreads();
+        if (e == 2) break;  // the trajectory is decided by an earlier try
         if (e) {
           if (tid == 0) atomicExch(kp.error, 1);
           r = S_CAPPED;
+        } else if (may_spec && !spec && L.tries >= kp.spec_from) {
+          try_record();
         }
       }
       if (r == S_CONTINUE) {
@@ -577,13 +602,7 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
         if (tid == 0) write_result(K, L, 2, 0.0, sm.blk);
         break;
       }
-      if (may_spec && L.tries >= kp.spec_from) {  // hand the remaining tries to the speculative phase
-        if (tid == 0) sm.idx = record_spec(kp, np, L) ? 1ull : 0ull;
-        __syncthreads();
-        const bool recorded = sm.idx != 0;
-        __syncthreads();
-        if (recorded) break;
-      }
+      if (may_spec && L.tries >= kp.spec_from) try_record();
       load_init<T, GAS>(L, lane_setup<T, GAS>(Kg, L.j));
       L.mode = M_RESTART;
       list_n = -1;
