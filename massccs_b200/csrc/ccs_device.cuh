@@ -1167,14 +1167,15 @@ template <typename T> __device__ __forceinline__ bool outside_box(const KParams 
 // kept.
 enum : int { M_IDLE = 0, M_INIT = 1, M_RESTART = 2, M_STEP = 3 };
 constexpr int BLOCK = 128;
-// Resident CTAs per SM the register allocation must allow.  Lane pass: 3.
-// Warp pass: molecules run 512 threads per SM (8 CTAs of 64 at <= 128
-// registers; measured 2.58 -> 2.07 s on the 1231-atom N2 workload, whose
-// warp pass is throughput-bound), atoms are left unconstrained (their warp
-// pass is bound by the latency of the longest trajectory), and so is the
-// FP64 parity mode (128 registers would spill).
+// Resident CTAs per SM the register allocation must allow.  Lane pass: 4 in
+// FP32 with a full warp per force evaluation (128 registers: the pass issues
+// on half of the cycles at 12 warps an SM, so the 16 pay more than the few
+// spilled words cost: n2_complex 199 -> 161 ms, he_assembly 343 -> 294; 5
+// spill into the loops), else 3.  The learned field's warp pass: molecules
+// run 512 threads per SM (8 CTAs of 64 at <= 128 registers), atoms are left
+// unconstrained.
 #ifndef CCS_LANE_MIN_BLOCKS
-#define CCS_LANE_MIN_BLOCKS 3
+#define CCS_LANE_MIN_BLOCKS(T, G) (sizeof(T) == 4 && (G) == 32 ? 4 : 3)
 #endif
 #ifndef CCS_WARP_MIN_BLOCKS
 #define CCS_WARP_MIN_BLOCKS(T, nt, gas) ((gas) == GAS_ATOM || sizeof(T) == 8 ? 1 : 512 / (nt))
@@ -1491,7 +1492,7 @@ __device__ __forceinline__ const KParams *ion_params_ptr(const KParams &kp, cons
 // MLP tile spans the CTA's 128 lanes; probes in the exact zone take the
 // exact path below as before.
 template <typename T, int G, int GAS, bool HASQ, bool BATCH, bool SURR = false>
-__global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS(T, G))
     traj_kernel(KParams kp, const KParams *__restrict__ kpg) {
   using S = Sites<GAS>;
   constexpr int NS = S::NS;
