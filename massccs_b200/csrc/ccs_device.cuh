@@ -108,7 +108,7 @@ struct KParams {
   uint32_t park_steps;
   int park_drained;                 // 1: park only once every trajectory has been taken
   int lcap;                         // warp pass: most entries of a candidate list
-  int wp_cap, wp_pack;              // warp pass: entries that the shared memory holds; 1: packed candidates too
+  int wp_cap, wp_pack;              // warp pass: list entries and packed candidates that the shared memory holds
   // batched ions: per-ion parameters (their rnd/status/omc/steps/visits point
   // at the ion's first trajectory) and the global index of each ion's first
   // trajectory (nions + 1 entries); unused by single-ion runs
@@ -794,6 +794,7 @@ __device__ __forceinline__ void eval_row(const KParams &kp, const T (&p)[GasShap
 constexpr int LCAP = 2048;  // least candidate-list entries kept in shared memory per CTA (the
                             // launch's kp.lcap, sized to the target's densest sphere, can be more)
 constexpr int LCAP_MAX = 8192;
+constexpr int WP_BLOCK = 512;   // the warp pass's packed list ends in whole blocks (at most 4 x 128 candidates)
 constexpr float LSKIN = 1.0f;  // A: the list's margin; reused while the probe moves less
 
 // Block-wide exclusive scan of len; total receives the block sum.  Ends
@@ -1336,11 +1337,10 @@ __device__ __noinline__ double lane_chi(const KParams *__restrict__ kpg, unsigne
   return one_minus_cos<T>(vref, vf);
 }
 
-// First half of a step: kick, drift (constrained for molecules), angle.
+// First half of a step: kick and drift (constrained for molecules).
 // inv_dt = 1 / L.dt (read for molecules).
 template <typename T, int GAS>
-__device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L, T inv_dt) {
-  using S = Sites<GAS>;
+__device__ __forceinline__ void first_half_move(const KParams &kp, LaneState<T> &L, T inv_dt) {
   const KConst<T> &kc = kconst<T>(kp);
   const T dt = L.dt;
   if constexpr (GAS == GAS_ATOM) {
@@ -1353,9 +1353,6 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L, T
       L.r1lo[k] = (t - L.r1[k]) - y;
       L.r1[k] = t;
     }
-    L.dtheta += angle3(L.r1, L.rold);
-#pragma unroll
-    for (int k = 0; k < 3; k++) L.rold[k] = L.r1[k];
   } else {
     // constrained Verlet, first half (System.cpp:1700-1739)
     const T d2 = sizeof(T) == 4 ? kc.d2 : T(kp.d_bond * kp.d_bond);
@@ -1387,13 +1384,24 @@ __device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L, T
       L.r2lo[k] = (t - L.r2[k]) - y;
       L.r2[k] = t;
     }
-    T rcm[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) rcm[k] = T(0.5) * (L.r1[k] + L.r2[k]);
-    L.dtheta += angle3(rcm, L.rold);
-#pragma unroll
-    for (int k = 0; k < 3; k++) L.rold[k] = rcm[k];
   }
+}
+
+// Component k of the (centre) position.
+template <typename T, int GAS> __device__ __forceinline__ T centre(const LaneState<T> &L, int k) {
+  return GAS == GAS_ATOM ? L.r1[k] : T(0.5) * (L.r1[k] + L.r2[k]);
+}
+// The angle that the step turned the centre by, into the running sum.
+template <typename T, int GAS> __device__ __forceinline__ void turn(LaneState<T> &L) {
+  const T c[3] = {centre<T, GAS>(L, 0), centre<T, GAS>(L, 1), centre<T, GAS>(L, 2)};
+  L.dtheta += angle3(c, L.rold);
+#pragma unroll
+  for (int k = 0; k < 3; k++) L.rold[k] = c[k];
+}
+template <typename T, int GAS>
+__device__ __forceinline__ void first_half(const KParams &kp, LaneState<T> &L, T inv_dt) {
+  first_half_move<T, GAS>(kp, L, inv_dt);
+  turn<T, GAS>(L);
 }
 
 enum : int { S_CONTINUE = 0, S_RETRY_ANGLE = 1, S_RETRY_ENERGY = 2, S_SCATTER = 3, S_CAPPED = 4 };
@@ -1405,14 +1413,11 @@ template <typename T> __device__ __forceinline__ bool step_leaves(const KParams 
   return outside_box(kp, L.rold);  // first_half left the (centre) position there
 }
 
-// Second half of a step and the exit tests (System.cpp:441-506, 835-940,
-// 1268-1387).  out = step_leaves(); L.U is read only when it is set.  The
-// centre-of-mass velocity for chi is exit_velocity's.
+// Second half of a step (System.cpp:441-506, 835-940, 1268-1387).
 template <typename T, int GAS>
-__device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, bool out) {
-  using S = Sites<GAS>;
+__device__ __forceinline__ void second_kick(const KParams &kp, LaneState<T> &L) {
   const KConst<T> &kc = kconst<T>(kp);
-  const T dt = L.dt, ke = T(AMUANGFS2_TO_KCAL_MOL);
+  const T dt = L.dt;
   if constexpr (GAS == GAS_ATOM) {
     const T kick = dt * kc.half_kconv_over_m1;
 #pragma unroll
@@ -1438,6 +1443,13 @@ __device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, b
   }
   L.stepcount++;
   L.nsteps++;
+}
+// Its exit tests.  out = step_leaves(); L.U is read only when it is set.  The
+// centre-of-mass velocity for chi is exit_velocity's.
+template <typename T, int GAS> __device__ __forceinline__ int exit_test(const KParams &kp, const LaneState<T> &L, bool out) {
+  using S = Sites<GAS>;
+  const KConst<T> &kc = kconst<T>(kp);
+  const T ke = T(AMUANGFS2_TO_KCAL_MOL);
   if (L.dtheta > T(1.5 * PI_D)) return S_RETRY_ANGLE;
   if (out) {
     T ek;
@@ -1457,6 +1469,11 @@ __device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, b
     return dE > kp.etol ? S_RETRY_ENERGY : S_SCATTER;
   }
   return L.stepcount >= kp.max_steps ? S_CAPPED : S_CONTINUE;
+}
+template <typename T, int GAS>
+__device__ __forceinline__ int second_half(const KParams &kp, LaneState<T> &L, bool out) {
+  second_kick<T, GAS>(kp, L);
+  return exit_test<T, GAS>(kp, L, out);
 }
 // Component k of the centre-of-mass velocity.
 template <typename T, int GAS> __device__ __forceinline__ T exit_velocity(const LaneState<T> &L, int k) {

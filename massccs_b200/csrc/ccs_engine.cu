@@ -265,10 +265,11 @@ int warp_shape(ccs_ctx *c, const WarpKernel &wk, KParams &k, size_t most_atoms, 
   k.wp_pack = 0;
   dyn = (size_t)(k.lcap + LCAP) * sizeof(int);
   if (!k.field.on) {
-    dyn = (size_t)k.wp_cap * sizeof(int);
-    const size_t packed = (size_t)k.wp_cap * (sizeof(float4) + (c->p.gas == CCS_GAS_CO2 ? 2 : 1) * sizeof(float2));
-    if (c->p.precision != CCS_PREC_FP64 && dyn + packed <= 58 * 1024) {
-      k.wp_pack = 1;
+    dyn = ((size_t)k.wp_cap * sizeof(int) + 15) / 16 * 16;
+    const int places = (k.wp_cap + WP_BLOCK - 1) / WP_BLOCK * WP_BLOCK;  // whole blocks
+    const size_t packed = (size_t)places * (sizeof(float4) + (c->p.gas == CCS_GAS_CO2 ? 2 : 1) * sizeof(float2));
+    if (c->p.precision != CCS_PREC_FP64 && dyn + packed <= 60 * 1024) {
+      k.wp_pack = places;
       dyn += packed;
     }
   }

@@ -31,14 +31,18 @@ template <int GAS, bool HASQ> struct Roles {
   static constexpr bool force(int r) { return ATOM ? r == 0 : r < 3; }
   static constexpr bool field(int r) { return HASQ && (ATOM ? r == 0 : GAS == GAS_N2 ? r == 2 : r == 3); }
   static constexpr bool grad(int r) { return HASQ && r == N - 1; }
+  // the first role of the same shape (a molecule's two like atoms): the two
+  // run one code, since instruction fetch is what a full SM waits for
+  static constexpr int code(int r) { return GAS == GAS_N2 && r == 1 ? 0 : GAS == GAS_CO2 && r == 2 ? 0 : r; }
 };
 
 // One candidate's terms of role R, in the order and with the roundings of
 // visit_atom.  LJ: the candidate may be inside the LJ cutoff (a group of
 // candidates that all lie beyond it adds exact zeros, and is passed by).
+// p, kq: position and charge factor of the role's site.
 template <typename T, int GAS, bool HASQ, int R, bool LJ>
-__device__ __forceinline__ void visit_role(const KParams &kp, const T (&p)[3], const Atom<T> &a, bool dipf, T (&f)[3],
-                                           T (&E)[3], T (&G)[6]) {
+__device__ __forceinline__ void visit_role(const KParams &kp, const T (&p)[3], T kq, const Atom<T> &a, bool dipf,
+                                           T (&f)[3], T (&E)[3], T (&G)[6]) {
   using RO = Roles<GAS, HASQ>;
   constexpr int s = RO::site(R);
   constexpr int lj = site_lj<GAS>(s);
@@ -61,7 +65,7 @@ __device__ __forceinline__ void visit_role(const KParams &kp, const T (&p)[3], c
     if constexpr (RO::force(R) && site_coul<GAS>(s)) {
       T ir3c = Real<T>::fma(ir, ir2, -kc.rc3inv);
       if constexpr (s == GasShape<GAS>::DIP) ir3c = dipf ? ir3c : ir3s;
-      const T fc = in_c ? kc.kq[s] * a.q * ir3c : T(0);
+      const T fc = in_c ? kq * a.q * ir3c : T(0);
       f[0] += fc * dx; f[1] += fc * dy; f[2] += fc * dz;
     }
     if constexpr (RO::field(R) || RO::grad(R)) {
@@ -82,19 +86,23 @@ __device__ __forceinline__ void visit_role(const KParams &kp, const T (&p)[3], c
 }
 
 // Where a step's candidates are: packed in shared memory in list order
-// (FP32), or atoms of the global tables, by index or all of them.
-template <typename T> struct Cand {
-  const float4 *pos;   // packed x, y, z, q (nullptr: not packed)
+// (FP32; every address a shared one), or atoms of the global tables, by index
+// or all of them.
+enum : int { C_NONE = 0, C_PACK = 1, C_LIST = 2, C_ALL = 3 };
+struct Cand {
+  const float4 *pos;   // packed x, y, z, q; far atoms up to the end of the last block
   const float2 *ab, *abc;
-  const int *list;     // atom indices (nullptr: atom t is candidate t)
+  const int *list;     // atom indices
   const unsigned *ljm; // one bit per 32 candidates of this virtual warp: some may be inside the LJ cutoff
+  bool masked;         // ljm is valid (else every candidate may be)
   int m;
 };
 
-template <typename T, int GAS, bool PACK, bool LJ>
-__device__ __forceinline__ Atom<T> fetch(const KParams &kp, const Cand<T> &c, int t) {
+template <typename T, int GAS, int MODE, bool LJ>
+__device__ __forceinline__ Atom<T> fetch(const KParams &kp, const Cand &c, int t) {
   Atom<T> a;
-  if constexpr (PACK) {
+  a.A = a.B = a.Ac = a.Bc = T(0);
+  if constexpr (MODE == C_PACK) {
     const float4 q = c.pos[t];
     a.x = q.x; a.y = q.y; a.z = q.z; a.q = q.w;
     if constexpr (LJ) {
@@ -102,9 +110,8 @@ __device__ __forceinline__ Atom<T> fetch(const KParams &kp, const Cand<T> &c, in
       a.A = ab.x; a.B = ab.y;
       if constexpr (GAS == GAS_CO2) { const float2 v = c.abc[t]; a.Ac = v.x; a.Bc = v.y; }
     }
-    return a;
   } else {
-    const int i = c.list ? c.list[t] : t;
+    const int i = MODE == C_LIST ? c.list[t] : t;
     if constexpr (sizeof(T) == 4) {
       const float4 q = __ldg(&kp.xyzq32[i]);
       a.x = q.x; a.y = q.y; a.z = q.z; a.q = q.w;
@@ -122,8 +129,18 @@ __device__ __forceinline__ Atom<T> fetch(const KParams &kp, const Cand<T> &c, in
         if constexpr (GAS == GAS_CO2) { const double2 v = kp.abc64[i]; a.Ac = v.x; a.Bc = v.y; }
       }
     }
-    return a;
   }
+  return a;
+}
+
+// An atom whose every term is an exact zero: it fills a lane's place past the
+// end of the candidates, so that the last ones run side by side as well
+// (one at a time they cost up to three full latencies a step).
+template <typename T> __device__ __forceinline__ Atom<T> far_atom() {
+  Atom<T> a;
+  a.x = T(1e18);
+  a.y = a.z = a.q = a.A = a.B = a.Ac = a.Bc = T(0);
+  return a;
 }
 
 // How many of a lane's candidates are in flight at once.  A lone warp per
@@ -131,47 +148,67 @@ __device__ __forceinline__ Atom<T> fetch(const KParams &kp, const Cand<T> &c, in
 // other candidates' work.
 constexpr int WP_ILP = 4;
 
-// Role R's sums over the candidates of virtual thread vt (vt, vt + NT, ...).
-template <typename T, int GAS, bool HASQ, int R, int NT, bool PACK>
-__device__ __forceinline__ void role_visits(const KParams &kp, const T (&p)[3], const Cand<T> &c, int vt, T (&f)[3],
+// Role R's sums over the candidates of virtual thread vt (vt, vt + NT, ...),
+// WP_ILP of them side by side.  The packed list ends in far atoms, so its
+// blocks are all whole; the others mask their last block.
+template <typename T, int GAS, bool HASQ, int R, int NT, int MODE>
+__device__ __forceinline__ void role_visits(const KParams &kp, const T (&p)[3], T kq, const Cand &c, int vt, T (&f)[3],
                                             T (&E)[3], T (&G)[6]) {
   using RO = Roles<GAS, HASQ>;
   constexpr bool HASLJ = RO::force(R) && site_lj<GAS>(RO::site(R)) != 0;
   constexpr bool PF = sizeof(T) == 4 && GAS == GAS_CO2;  // see visit_atom's DIPF
-  const int cnt = vt < c.m ? (c.m - vt + NT - 1) / NT : 0;
-  int k = 0, t = vt;
-  for (; k + WP_ILP <= cnt; k += WP_ILP, t += WP_ILP * NT) {
-    const bool lj = HASLJ && (!c.ljm || ((c.ljm[k >> 5] >> (k & 31)) & ((1u << WP_ILP) - 1u)) != 0);
-    if (lj) {
-      Atom<T> a[WP_ILP];
-#pragma unroll
-      for (int i = 0; i < WP_ILP; i++) a[i] = fetch<T, GAS, PACK, HASLJ>(kp, c, t + i * NT);
-#pragma unroll
-      for (int i = 0; i < WP_ILP; i++) visit_role<T, GAS, HASQ, R, HASLJ>(kp, p, a[i], PF, f, E, G);
-    } else if (HASQ) {
-      Atom<T> a[WP_ILP];
-#pragma unroll
-      for (int i = 0; i < WP_ILP; i++) a[i] = fetch<T, GAS, PACK, false>(kp, c, t + i * NT);
-#pragma unroll
-      for (int i = 0; i < WP_ILP; i++) visit_role<T, GAS, HASQ, R, false>(kp, p, a[i], PF, f, E, G);
-    }
-  }
+  constexpr bool TAILF = PF && NT == 32 && RO::force(R) && RO::site(R) == GasShape<GAS>::DIP;
+  const int wbase = vt & ~31;  // the same count of rounds for the whole warp
+  const int rounds = wbase < c.m ? (c.m - wbase + NT - 1) / NT : 0;
+  const int cnt = (MODE != C_PACK || TAILF) && vt < c.m ? (c.m - vt + NT - 1) / NT : 0;
 #pragma unroll 1
-  for (; k < cnt; k++, t += NT) {
-    const Atom<T> a = fetch<T, GAS, PACK, HASLJ>(kp, c, t);
-    visit_role<T, GAS, HASQ, R, HASLJ>(kp, p, a, PF && !(NT == 32 && (cnt & 1) && k == cnt - 1), f, E, G);
+  for (int k = 0, t = vt; k < rounds; k += WP_ILP, t += WP_ILP * NT) {
+    Atom<T> a[WP_ILP];
+    bool lj = false;
+    if constexpr (HASLJ) lj = !c.masked || ((c.ljm[k >> 5] >> (k & 31)) & ((1u << WP_ILP) - 1u)) != 0;
+    if (HASLJ && lj) {
+#pragma unroll
+      for (int i = 0; i < WP_ILP; i++) {
+        if constexpr (MODE != C_PACK) a[i] = far_atom<T>();
+        if (MODE == C_PACK || k + i < cnt) a[i] = fetch<T, GAS, MODE, HASLJ>(kp, c, t + i * NT);
+      }
+#pragma unroll
+      for (int i = 0; i < WP_ILP; i++)
+        visit_role<T, GAS, HASQ, R, HASLJ>(kp, p, kq, a[i], PF && !(TAILF && (cnt & 1) && k + i == cnt - 1), f, E, G);
+    } else if constexpr (HASQ) {
+#pragma unroll
+      for (int i = 0; i < WP_ILP; i++) {
+        if constexpr (MODE != C_PACK) a[i] = far_atom<T>();
+        if (MODE == C_PACK || k + i < cnt) a[i] = fetch<T, GAS, MODE, false>(kp, c, t + i * NT);
+      }
+#pragma unroll
+      for (int i = 0; i < WP_ILP; i++)
+        visit_role<T, GAS, HASQ, R, false>(kp, p, kq, a[i], PF && !(TAILF && (cnt & 1) && k + i == cnt - 1), f, E, G);
+    }
   }
 }
 
 // The sums of one role over its candidates, reduced over the warp into row
 // (the part of it that is the role's).
-template <typename T, int GAS, bool HASQ, int R> __device__ __forceinline__ void role_reduce(const T (&f)[3], const T (&E)[3],
-                                                                                            const T (&G)[6], int lane, T *row) {
+template <typename T, int GAS, bool HASQ, int R>
+__device__ __forceinline__ void role_reduce(int role, const T (&f)[3], const T (&E)[3], const T (&G)[6], int lane, T *row) {
   using RO = Roles<GAS, HASQ>;
   constexpr int K0 = RO::k0(R), K1 = RO::k1(R);
+  if (RO::force(R)) row += 3 * (role - R);  // a role that shares this code: its own site's entries
   warp_sum_rows<K1 - K0, T>(
       [&](int k) { return k >= Row<GAS>::G ? G[(k - Row<GAS>::G) % 6] : k >= Row<GAS>::E ? E[(k - Row<GAS>::E) % 3] : f[k % 3]; },
       K0, lane, row);
+}
+
+// Far atoms in the packed places from n to the end of its last block.
+template <int GAS, int NT>
+__device__ __forceinline__ void pack_end(int n, int tid, int nthreads, float4 *pos, float2 *ab, float2 *abc) {
+  const int end = (n + WP_ILP * NT - 1) / (WP_ILP * NT) * (WP_ILP * NT);
+  for (int t = n + tid; t < end; t += nthreads) {
+    pos[t] = make_float4(1e18f, 0.f, 0.f, 0.f);
+    ab[t] = make_float2(0.f, 0.f);
+    if constexpr (GAS == GAS_CO2) abc[t] = make_float2(0.f, 0.f);
+  }
 }
 
 // Atom i as packed candidate t.
@@ -184,43 +221,56 @@ __device__ __forceinline__ void pack_atom(const KParams &kp, int i, int t, float
   }
 }
 
-// This warp's role in one force evaluation.
+// This warp's role in one force evaluation.  sa: atomic gases, a small
+// target's atoms of this virtual thread, held in registers (C_NONE: they are
+// the candidates).
 template <typename T, int GAS, bool HASQ, int NT, int R = 0>
 __device__ __forceinline__ void step_visits(const KParams &kp, int role, const T (&p)[GasShape<GAS>::NS][3],
-                                            unsigned actbits, const Cand<T> &c, int vt, T (&f)[3], T (&E)[3], T (&G)[6]) {
+                                            unsigned actbits, int mode, const Cand &c, const Atom<T> (&sa)[2], int vt,
+                                            T (&f)[3], T (&E)[3], T (&G)[6]) {
   using RO = Roles<GAS, HASQ>;
-  if constexpr (R < RO::N) {
-    if (role == R) {
-      constexpr int s = RO::site(R);
+  if constexpr (R < RO::N && RO::code(R < RO::N ? R : 0) != R) {
+    step_visits<T, GAS, HASQ, NT, R + 1>(kp, role, p, actbits, mode, c, sa, vt, f, E, G);
+  } else if constexpr (R < RO::N) {
+    if (RO::code(role) == R) {
+      const int s = RO::site(R) + (role - R);
       if (!((actbits >> s) & 1u) || (!RO::force(R) && !kp.dip_on)) return;  // the site feels nothing
-      if constexpr (sizeof(T) == 4) {
-        if (c.pos) { role_visits<T, GAS, HASQ, R, NT, true>(kp, p[s], c, vt, f, E, G); return; }
+      T ps[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        ps[k] = p[RO::site(R)][k];
+#pragma unroll
+        for (int q = R + 1; q < RO::N; q++)
+          if (RO::code(q) == R && role == q) ps[k] = p[RO::site(q)][k];
       }
-      role_visits<T, GAS, HASQ, R, NT, false>(kp, p[s], c, vt, f, E, G);
+      const T kq = kconst<T>(kp).kq[RO::site(R)];  // roles of one code: equal charges
+      if constexpr (GAS == GAS_ATOM) {
+        if (mode == C_NONE) {
+          visit_role<T, GAS, HASQ, R, true>(kp, ps, kq, sa[0], false, f, E, G);
+          if (c.m > NT) visit_role<T, GAS, HASQ, R, true>(kp, ps, kq, sa[1], false, f, E, G);
+          return;
+        }
+      }
+      if constexpr (sizeof(T) == 4) {
+        if (mode == C_PACK) { role_visits<T, GAS, HASQ, R, NT, C_PACK>(kp, ps, kq, c, vt, f, E, G); return; }
+      }
+      if (mode == C_LIST) role_visits<T, GAS, HASQ, R, NT, C_LIST>(kp, ps, kq, c, vt, f, E, G);
+      else role_visits<T, GAS, HASQ, R, NT, C_ALL>(kp, ps, kq, c, vt, f, E, G);
     } else {
-      step_visits<T, GAS, HASQ, NT, R + 1>(kp, role, p, actbits, c, vt, f, E, G);
+      step_visits<T, GAS, HASQ, NT, R + 1>(kp, role, p, actbits, mode, c, sa, vt, f, E, G);
     }
   }
 }
 template <typename T, int GAS, bool HASQ, int R = 0>
 __device__ __forceinline__ void step_reduce(int role, const T (&f)[3], const T (&E)[3], const T (&G)[6], int lane, T *row) {
-  if constexpr (R < Roles<GAS, HASQ>::N) {
-    if (role == R) role_reduce<T, GAS, HASQ, R>(f, E, G, lane, row);
+  using RO = Roles<GAS, HASQ>;
+  if constexpr (R < RO::N && RO::code(R < RO::N ? R : 0) != R) {
+    step_reduce<T, GAS, HASQ, R + 1>(role, f, E, G, lane, row);
+  } else if constexpr (R < RO::N) {
+    if (RO::code(role) == R) role_reduce<T, GAS, HASQ, R>(role, f, E, G, lane, row);
     else step_reduce<T, GAS, HASQ, R + 1>(role, f, E, G, lane, row);
   }
 }
-
-// Shared memory of the pass besides the candidate lists.
-template <typename T, int GAS, int NT> struct WarpShared {
-  static constexpr int NW = NT / 32;
-  static constexpr int ROWP = (Row<GAS>::N + 3) / 4 * 4;
-  alignas(16) T red[2][NW][ROWP];  // reduced sums per virtual warp, alternating
-  unsigned ljm[NW][LCAP_MAX / 32 / NW / 32 > 0 ? LCAP_MAX / 32 / NW / 32 : 1];
-  int wsum[NW];
-  unsigned long long blk[8];
-  unsigned long long idx;
-  int kind, stop;
-};
 
 // Exclusive scan of the run lengths of the NT threads of role 0 (every thread
 // of the CTA calls; the others pass len = 0 and get no position).  Two
@@ -275,6 +325,139 @@ __device__ __forceinline__ uint32_t for_chunks(const KParams &kp, T cx, T cy, T 
   return nvis;
 }
 
+// Shared memory of the pass besides the candidate lists.
+template <typename T, int GAS, int NT> struct WarpShared {
+  static constexpr int NW = NT / 32;
+  static constexpr int ROWP = (Row<GAS>::N + 3) / 4 * 4;
+  alignas(16) T red[2][NW][ROWP];  // reduced sums per virtual warp, alternating
+  unsigned ljm[NW][LCAP_MAX / 32 / NW / 32 > 0 ? LCAP_MAX / 32 / NW / 32 : 1];
+  int wsum[NW];
+  unsigned long long blk[8];
+  unsigned long long idx;
+  int kind, stop;
+};
+
+// The rounded square root of x without a branch (the usual call has one for
+// the ends of the range): a Newton step from the approximate reciprocal root,
+// then Tuckerman's test on the exact remainder (Agarwal et al. 1986) moves
+// the result to the neighbour if that is nearer.  For 1e-18 <= x <= 1e18.
+__device__ __forceinline__ float sqrt_mid(float x) {
+  const float y = rsqrtf(x);
+  float s = __fmul_rn(x, y);
+  s = __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+  const float r = __fmaf_rn(-s, s, x);
+  const float up = __int_as_float(__float_as_int(s) + 1), dn = __int_as_float(__float_as_int(s) - 1);
+  return r > __fmul_rn(s, up - s) ? up : r <= -__fmul_rn(s, s - dn) ? dn : s;
+}
+
+// angle3 of a usual step, without branches; wide: it is not the small angle
+// of the series (or too small for the root), and is left to angle3.
+template <typename T> __device__ __forceinline__ T small_angle(const T a[3], const T b[3], bool &wide) {
+  if constexpr (sizeof(T) == 8) {
+    wide = false;
+    return angle3(a, b);
+  } else {
+    const float cx = a[1] * b[2] - a[2] * b[1], cy = a[2] * b[0] - a[0] * b[2],
+                cz = a[0] * b[1] - a[1] * b[0];
+    const float c2 = cx * cx + cy * cy + cz * cz, cs = dot3(a, b);
+    const float sn = sqrt_mid(c2);
+    wide = !((c2 >= 1e-18f) & (c2 <= 1e18f) & (cs > 0.f) & (sn < 0.125f * cs));
+    const float t = __fdividef(sn, cs), t2 = t * t;
+    return t * (1.f + t2 * (-1.f / 3.f + t2 * (1.f / 5.f + t2 * (-1.f / 7.f + t2 * (1.f / 9.f)))));
+  }
+}
+
+// The sums of a step from the virtual warps' partials, in a fixed order, and
+// the forces from them.
+template <typename T, int GAS, bool HASQ, int NT>
+__device__ __forceinline__ void step_forces(const KParams &kp, const T (*red)[WarpShared<T, GAS, NT>::ROWP],
+                                            const bool (&act)[GasShape<GAS>::NS], LaneState<T> &L, T *sum) {
+#pragma unroll
+  for (int k = 0; k < Row<GAS>::forces(HASQ); k++) {
+    sum[k] = red[0][k];
+#pragma unroll
+    for (int q = 1; q < NT / 32; q++) sum[k] += red[q][k];
+  }
+  if constexpr (GAS == GAS_N2 && !HASQ) sum[6] = sum[7] = sum[8] = T(0);  // the centre has no terms
+  T fs[GasShape<GAS>::NS][3];
+  finish_row<T, GAS, HASQ>(kp, sum, act, fs);
+  absorb_forces<T, GAS>(kp, fs, L);
+}
+
+// Bounds that decide a step well inside the cutoffs without its exact reach
+// (a square root on the way to the forces): half the pair distance within
+// half a percent of its constrained value.
+template <typename T> struct StepBounds {
+  T offhi, hd2lo, hd2hi, rin2, rout2;
+};
+enum : int { F_OTHER = 0, F_TEST = 1, F_WIDE = 2 };
+
+// Usual steps, one after another: the probe inside the reach and the
+// reference grid, its candidates known (mode), no end of the try.  Few
+// branches, so that what is not on the way to the forces (the angle, the
+// tests) fills the latencies of what is.  One copy of the integrator for all
+// roles: every warp of the CTA computes the same bits and takes the same
+// turns.  Returns F_OTHER: a step whose move is done and which is not usual;
+// F_TEST: after a step, an exit test or the periodic check is due; F_WIDE:
+// the same with the step's angle still to do.
+template <typename T, int GAS, bool HASQ, int NT>
+__device__ __forceinline__ int usual_steps(int role, const KParams &kp, LaneState<T> &L, T inv_dt,
+                                           const StepBounds<T> &sb, int mode, bool small, const Cand &cd,
+                                           const Atom<T> (&sa)[2], const T (&list_c)[3], int vt, int lane, int v,
+                                           WarpShared<T, GAS, NT> &sm, int &red, unsigned &it) {
+  constexpr int NS = GasShape<GAS>::NS;
+  const KConst<T> &kc = kconst<T>(kp);
+  const bool all = !cd.masked;
+  for (;;) {
+    first_half_move<T, GAS>(kp, L, inv_dt);
+    const T c[3] = {centre<T, GAS>(L, 0), centre<T, GAS>(L, 1), centre<T, GAS>(L, 2)};
+    const T ex = fmax(fmax(kc.bb_lo[0] - c[0], c[0] - kc.bb_hi[0]), T(0));
+    const T ey = fmax(fmax(kc.bb_lo[1] - c[1], c[1] - kc.bb_hi[1]), T(0));
+    const T ez = fmax(fmax(kc.bb_lo[2] - c[2], c[2] - kc.bb_hi[2]), T(0));
+    const T fx = fmax(c[0] - kc.bb_lo[0], kc.bb_hi[0] - c[0]);
+    const T fy = fmax(c[1] - kc.bb_lo[1], kc.bb_hi[1] - c[1]);
+    const T fz = fmax(c[2] - kc.bb_lo[2], kc.bb_hi[2] - c[2]);
+    const T e2 = ex * ex + ey * ey + ez * ez, f2 = fx * fx + fy * fy + fz * fz;
+    const T dcx = c[0] - list_c[0], dcy = c[1] - list_c[1], dcz = c[2] - list_c[2];
+    const T moved2 = Real<T>::fma(dcz, dcz, Real<T>::fma(dcx, dcx, Real<T>::mul(dcy, dcy)));
+    const T ux = c[0] * kc.inv_a, uy = c[1] * kc.inv_b, uz = c[2] * kc.inv_c;
+    const T ax = fabs(c[0]), ay = fabs(c[1]), az = fabs(c[2]);
+    bool ok = (e2 <= sb.rin2) & (ax + sb.offhi < kc.ref_lim[0]) & (ay + sb.offhi < kc.ref_lim[1]) &
+              (az + sb.offhi < kc.ref_lim[2]);
+    // strictly inside the box and the ellipsoid, with room for another rounding of outside_box's sum
+    ok &= (ax < kc.lx) & (ay < kc.ly) & (az < kc.lz) & (ux * ux + uy * uy + uz * uz < T(1) - T(1e-6));
+    ok &= small | (all ? f2 <= sb.rin2 : (f2 > sb.rout2) & (moved2 <= T(LSKIN) * T(LSKIN)));
+    if constexpr (GAS != GAS_ATOM) {
+      const T hd[3] = {L.r1[0] - L.r2[0], L.r1[1] - L.r2[1], L.r1[2] - L.r2[2]};
+      const T hd2 = dot3(hd, hd);
+      ok &= (hd2 >= sb.hd2lo) & (hd2 <= sb.hd2hi);
+    }
+    if (!ok) return F_OTHER;
+    bool wide;
+    const T ang = small_angle(c, L.rold, wide);
+    T p[NS][3];
+    site_positions<T, GAS>(L, p);
+    T f[3] = {T(0), T(0), T(0)}, E[3] = {T(0), T(0), T(0)}, G[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+    step_visits<T, GAS, HASQ, NT>(kp, role, p, (1u << NS) - 1u, mode, cd, sa, vt, f, E, G);
+    step_reduce<T, GAS, HASQ>(role, f, E, G, lane, sm.red[red][v]);
+    __syncthreads();
+    bool act[NS];
+#pragma unroll
+    for (int k = 0; k < NS; k++) act[k] = true;
+    T sum[Row<GAS>::N];
+    step_forces<T, GAS, HASQ, NT>(kp, sm.red[red], act, L, sum);
+    red ^= 1;
+    L.nvis += (uint32_t)cd.m;
+    second_kick<T, GAS>(kp, L);
+    it++;
+    if (wide) return F_WIDE;
+    L.dtheta += ang;
+#pragma unroll
+    for (int k = 0; k < 3; k++) L.rold[k] = c[k];
+    if ((L.dtheta > T(1.5 * PI_D)) | (L.stepcount >= kp.max_steps) | ((it & 255u) == 0)) return F_TEST;
+  }
+}
+
 // The sites' energies of a step that begins or ends a try, one warp per
 // virtual warp (the lead role's) in the order of the force sums, into
 // row[v][U..U + NS) of the reduction buffer.  Out of line: once or twice a try.
@@ -316,15 +499,14 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
   constexpr int NS = S::NS, NW = NT / 32, NTHREADS = WarpShape<T, GAS, HASQ, NT>::THREADS;
   constexpr bool PACKS = sizeof(T) == 4;
   constexpr bool RF = sizeof(T) == 4 && GAS != GAS_ATOM && NT != 32 && !BATCH;  // see column_run
-  constexpr int NF = Row<GAS>::forces(HASQ);
   __shared__ WarpShared<T, GAS, NT> sm;
   __shared__ __align__(16) unsigned char sm_kp[BATCH ? sizeof(KParams) : 16];  // this trajectory's ion
   extern __shared__ __align__(16) unsigned char dyn[];
   // candidate list: indices, then (kp.wp_pack) the packed candidates in list order
   int *const sm_list = reinterpret_cast<int *>(dyn);
   float4 *const sm_pos = reinterpret_cast<float4 *>(dyn + (((size_t)kp.wp_cap * 4 + 15) & ~size_t(15)));
-  float2 *const sm_ab = reinterpret_cast<float2 *>(sm_pos + kp.wp_cap);
-  float2 *const sm_abc = sm_ab + kp.wp_cap;
+  float2 *const sm_ab = reinterpret_cast<float2 *>(sm_pos + kp.wp_pack);
+  float2 *const sm_abc = sm_ab + kp.wp_pack;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   // the roles of a virtual warp sit on different sub-partitions; a second
   // virtual warp starts two further on, so light and heavy roles mix
@@ -397,10 +579,33 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
     // A target of at most two atoms per virtual thread is all candidates at every step
     const bool small = K.natoms <= 2 * NT;
     const bool packs = PACKS && kp.wp_pack;
-    if (packs && small) {
+    // its atoms stay in registers (atomic gases) or, as without cutoffs, packed
+    const bool insmall = GAS == GAS_ATOM && small;
+    const bool packall = packs && !insmall && (small || K.allpairs) && K.natoms <= kp.wp_cap;
+    Atom<T> sa[2] = {far_atom<T>(), far_atom<T>()};
+    Cand cd{sm_pos, sm_ab, sm_abc, sm_list, sm.ljm[v], false, 0};
+    if (insmall) {
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+        if (vt + i * NT < K.natoms) sa[i] = fetch<T, GAS, C_ALL, true>(K, cd, vt + i * NT);
+    }
+    if (packall) {
       for (int t = tid; t < K.natoms; t += NTHREADS) pack_atom<T, GAS>(K, t, t, sm_pos, sm_ab, sm_abc);
+      pack_end<GAS, NT>(K.natoms, tid, NTHREADS, sm_pos, sm_ab, sm_abc);
       __syncthreads();
     }
+    StepBounds<T> sb;
+    {
+      const T offm = GAS == GAS_ATOM ? T(0) : T(0.5) * T(sqrt(kc.d2)), offlo = offm * T(0.995);
+      sb.offhi = offm * T(1.005);
+      sb.hd2lo = T(4) * offlo * offlo;
+      sb.hd2hi = T(4) * sb.offhi * sb.offhi;
+      const T rin = K.allpairs ? T(INFINITY) : kc.reach + offlo, rout = kc.reach + sb.offhi + T(0.01);
+      sb.rin2 = rin * rin;
+      sb.rout2 = rout * rout;
+    }
+    int mode = C_NONE;
+    bool usual = false;  // the last step was near: the next may be a usual one
     int list_n = -1;  // this trajectory's candidate list (none yet)
     T list_c[3] = {T(0), T(0), T(0)};
     T inv_dt = Real<T>::div(T(1), L.dt);
@@ -438,41 +643,54 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
           try_record();
         }
       }
+      if (r == S_CONTINUE && usual && L.mode == M_STEP) {
+        const int u = usual_steps<T, GAS, HASQ, NT>(role, K, L, inv_dt, sb, mode, small, cd, sa, list_c, vt, lane, v, sm,
+                                                    red, it);
+        if (u == F_WIDE) turn<T, GAS>(L);
+        if (u != F_OTHER) {
+          it--;  // the loop's own count
+          r = exit_test<T, GAS>(K, L, false);
+          if (r == S_CONTINUE) continue;
+        }
+      }
       if (r == S_CONTINUE) {
         bool out = false;
         if (L.mode == M_STEP) {
-          first_half<T, GAS>(K, L, inv_dt);
+          if (!usual) first_half_move<T, GAS>(K, L, inv_dt);
+          turn<T, GAS>(L);
           out = step_leaves(K, L);
         }
+        usual = false;
         const bool want_u = L.mode == M_INIT || out;
         L.U = T(0);
-        T p[NS][3], fs[NS][3];
+        T p[NS][3];
         site_positions<T, GAS>(L, p);
+        const T cx = p[S::cs][0], cy = p[S::cs][1], cz = p[S::cs][2];
+        const T ex = fmax(fmax(kc.bb_lo[0] - cx, cx - kc.bb_hi[0]), T(0));
+        const T ey = fmax(fmax(kc.bb_lo[1] - cy, cy - kc.bb_hi[1]), T(0));
+        const T ez = fmax(fmax(kc.bb_lo[2] - cz, cz - kc.bb_hi[2]), T(0));
+        const T fx = fmax(cx - kc.bb_lo[0], kc.bb_hi[0] - cx);
+        const T fy = fmax(cy - kc.bb_lo[1], kc.bb_hi[1] - cy);
+        const T fz = fmax(cz - kc.bb_lo[2], kc.bb_hi[2] - cz);
+        const T e2 = ex * ex + ey * ey + ez * ez, f2 = fx * fx + fy * fy + fz * fz;
+        const T dcx = cx - list_c[0], dcy = cy - list_c[1], dcz = cz - list_c[2];
+        const T moved2 = Real<T>::fma(dcz, dcz, Real<T>::fma(dcx, dcx, Real<T>::mul(dcy, dcy)));
+        const bool keep = list_n >= 0 && !(moved2 > T(LSKIN) * T(LSKIN));
         unsigned actbits;
-        if (probe_near<T, GAS>(K, p, actbits)) {
-          bool act[NS];
-#pragma unroll
-          for (int s = 0; s < NS; s++) act[s] = (actbits >> s) & 1u;
+        bool chunked = false;
+        T R = T(0);
+        cd.m = K.natoms;
+        const bool near = probe_near<T, GAS>(K, p, actbits);
+        if (near) {
           const T off = site_offset<T, GAS>(p);
-          const T R = K.allpairs ? T(INFINITY) : kc.reach + off + T(1e-3);
-          const T cx = p[S::cs][0], cy = p[S::cs][1], cz = p[S::cs][2];
-          const T ex = fmax(fmax(kc.bb_lo[0] - cx, cx - kc.bb_hi[0]), T(0));
-          const T ey = fmax(fmax(kc.bb_lo[1] - cy, cy - kc.bb_hi[1]), T(0));
-          const T ez = fmax(fmax(kc.bb_lo[2] - cz, cz - kc.bb_hi[2]), T(0));
-          const T fx = fmax(cx - kc.bb_lo[0], kc.bb_hi[0] - cx);
-          const T fy = fmax(cy - kc.bb_lo[1], kc.bb_hi[1] - cy);
-          const T fz = fmax(cz - kc.bb_lo[2], kc.bb_hi[2] - cz);
-          Cand<T> cd{nullptr, sm_ab, sm_abc, nullptr, nullptr, 0};
-          bool chunked = false;
-          if (small || fx * fx + fy * fy + fz * fz <= R * R) {
+          R = K.allpairs ? T(INFINITY) : kc.reach + off + T(1e-3);
+          if (small || f2 <= R * R) {
             // the whole target inside the reach sphere, or a small target:
             // every atom is a candidate (the cutoff tests are exact)
-            cd.m = K.natoms;
-            if (packs && small) cd.pos = sm_pos;
-          } else if (ex * ex + ey * ey + ez * ez <= R * R) {
-            const T dcx = cx - list_c[0], dcy = cy - list_c[1], dcz = cz - list_c[2];
-            const T moved2 = Real<T>::fma(dcz, dcz, Real<T>::fma(dcx, dcx, Real<T>::mul(dcy, dcy)));
-            if (list_n < 0 || moved2 > T(LSKIN) * T(LSKIN)) {
+            mode = insmall ? C_NONE : packall ? C_PACK : C_ALL;
+            cd.masked = false;
+          } else if (e2 <= R * R) {
+            if (!keep) {
               // rebuild the list for the sphere of radius R + LSKIN around the centre
               const T RL = R + T(LSKIN);
               int i0, j0, nj;
@@ -509,27 +727,34 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
                   if (__any_sync(0xffffffffu, in) && lane == 0)
                     atomicOr(&sm.ljm[g % NW][g / NW >> 5], 1u << (g / NW & 31));
                 }
+                if (packs) pack_end<GAS, NT>(list_n, tid, NTHREADS, sm_pos, sm_ab, sm_abc);
                 __syncthreads();
               }
             }
-            if (list_n >= 0) {
-              cd.list = sm_list;
-              cd.ljm = sm.ljm[v];
-              cd.m = list_n;
-              if (packs) cd.pos = sm_pos;
-            } else {
-              chunked = true;
-            }
+            mode = packs ? C_PACK : C_LIST;
+            cd.masked = true;
+            cd.m = list_n;
+            chunked = list_n < 0;
+          } else {
+            mode = C_ALL;
+            cd.m = 0;  // no atom in reach
           }
+        }
+        if (near) {
+          bool act[NS];
+#pragma unroll
+          for (int s = 0; s < NS; s++) act[s] = (actbits >> s) & 1u;
           T af[3] = {T(0), T(0), T(0)}, aE[3] = {T(0), T(0), T(0)}, aG[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
           uint32_t nvis;
           if (chunked) {
             nvis = for_chunks<T, NT, RF>(K, cx, cy, cz, R, lead, lane, v, sm_list, lcap, sm.wsum, [&](int *l, int n) {
-              Cand<T> cc{nullptr, nullptr, nullptr, l, nullptr, n};
-              step_visits<T, GAS, HASQ, NT>(K, role, p, actbits, cc, vt, af, aE, aG);
+              Cand cc = cd;
+              cc.masked = false;
+              cc.m = n;
+              step_visits<T, GAS, HASQ, NT>(K, role, p, actbits, C_LIST, cc, sa, vt, af, aE, aG);
             });
           } else {
-            step_visits<T, GAS, HASQ, NT>(K, role, p, actbits, cd, vt, af, aE, aG);
+            step_visits<T, GAS, HASQ, NT>(K, role, p, actbits, mode, cd, sa, vt, af, aE, aG);
             nvis = (uint32_t)cd.m;
           }
           T *const row = sm.red[red][v];
@@ -543,20 +768,12 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
               for (int k = 0; k < 3; k++) ps.p[s][k] = p[s][k];
             }
             if (chunked) __syncthreads();  // the list is rewritten by the energy's chunks
-            warp_energy<T, GAS, HASQ, NT, RF>(Kg, ps, chunked, cx, cy, cz, R, chunked || cd.list ? sm_list : nullptr, cd.m,
+            warp_energy<T, GAS, HASQ, NT, RF>(Kg, ps, chunked, cx, cy, cz, R, chunked || cd.masked ? sm_list : nullptr, cd.m,
                                           lcap, lead, lane, v, sm.wsum, row);
           }
           __syncthreads();
-          // every thread sums the virtual warps' partials in the same fixed order
           T sum[Row<GAS>::N];
-#pragma unroll
-          for (int k = 0; k < NF; k++) {
-            sum[k] = sm.red[red][0][k];
-#pragma unroll
-            for (int q = 1; q < NW; q++) sum[k] += sm.red[red][q][k];
-          }
-          if constexpr (GAS == GAS_N2 && !HASQ) sum[6] = sum[7] = sum[8] = T(0);  // the centre has no terms
-          finish_row<T, GAS, HASQ>(K, sum, act, fs);
+          step_forces<T, GAS, HASQ, NT>(K, sm.red[red], act, L, sum);
           if (want_u) {
 #pragma unroll
             for (int k = Row<GAS>::U; k < Row<GAS>::N; k++) {
@@ -568,11 +785,13 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
           }
           red ^= 1;
           L.nvis += nvis;
+          usual = !chunked && cd.m > 0;
         } else {
+          T fs[NS][3];
 #pragma unroll
           for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = T(0);
+          absorb_forces<T, GAS>(K, fs, L);
         }
-        absorb_forces<T, GAS>(K, fs, L);
         if (L.mode == M_INIT) { L.Ei += L.U; L.mode = M_STEP; continue; }
         if (L.mode == M_RESTART) { L.mode = M_STEP; continue; }
         r = second_half<T, GAS>(K, L, out);
@@ -606,6 +825,7 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
       load_init<T, GAS>(L, lane_setup<T, GAS>(Kg, L.j));
       L.mode = M_RESTART;
       list_n = -1;
+      usual = false;
     }
     // a parked trajectory has ended (or its record is published): one fewer running
     if (tid == 0 && !spec && may_spec) {
