@@ -330,12 +330,22 @@ int arm_deadline(ccs_ctx *c, unsigned long long *word, cudaStream_t s) {
 }
 
 // Grid and trajectories per warp of the lane pass.  A warp evaluates the
-// forces of its probes one after another, so fewer trajectories than lanes
-// in the resident warps are spread over all of them, the fewest per warp.
-void lane_shape(const ccs_ctx *c, size_t n, int per_sm, size_t &grid, int &width) {
-  const size_t warps_cta = BLOCK / 32;
+// forces of its probes one after another, so a run is spread over all resident
+// warps before any takes a second trajectory, and over about four rounds of
+// them before the warps fill up: the rounds even out the trajectories'
+// lengths, and a narrower warp ends its last ones sooner.  Measured, lane
+// pass, against one round: n2_complex (20,000 trajectories) 160 -> 123 ms,
+// he_assembly (60,000) 293 -> 238, n2_protein_3k 30 -> 20; 8 and 16 rounds give
+// another 1-3 % there but cost 20-60 % on the 60-atom cage, whose steps are
+// mostly integration (a full warp's).  Groups of G lanes work on 32 / G probes
+// at once, so there are at least as many.  The learned field's tiles span the
+// CTA's 128 lanes: it fills its warps (G = 0).
+void lane_shape(const ccs_ctx *c, size_t n, int per_sm, int G, size_t &grid, int &width) {
+  const size_t warps_cta = BLOCK / 32, rounds = 4;
   grid = (size_t)std::max(per_sm, 1) * c->sm_count;
-  width = (int)std::min<size_t>(32, std::max<size_t>(1, (n + grid * warps_cta - 1) / (grid * warps_cta)));
+  const int groups = G > 0 ? 32 / G : 32;
+  const size_t share = (n + grid * warps_cta * rounds - 1) / (grid * warps_cta * rounds);
+  width = (int)std::min<size_t>(32, (share + groups - 1) / groups * groups);
   grid = std::min(grid, std::max<size_t>(1, (n + warps_cta * width - 1) / (warps_cta * width)));
 }
 
@@ -361,7 +371,7 @@ int run_device(ccs_ctx *c, size_t n, const double *d_rnd, size_t stride, int8_t 
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, block, dyn));
   size_t grid = 0;
-  lane_shape(c, n, per_sm, grid, k.lane_width);
+  lane_shape(c, n, per_sm, surr ? 0 : G, grid, k.lane_width);
   k.deadline = c->d_work + 8;
   // longest-expected-first processing order (a radix sort of the length keys)
   if (n > 1 && c->p.schedule == 1) {
@@ -574,7 +584,7 @@ int run_batch_device(ccs_ctx *lead, ccs_ctx *const *ions, size_t nions, const si
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, BLOCK, 0));
   size_t grid = 0;
-  lane_shape(lead, total, per_sm, grid, k.lane_width);
+  lane_shape(lead, total, per_sm, Gb, grid, k.lane_width);
   CK(cudaEventRecord(lead->ev[5], s));
   fn<<<(unsigned)grid, BLOCK, 0, s>>>(k, lead->d_kparams);
   CK(cudaGetLastError());
@@ -1290,7 +1300,7 @@ extern "C" int ccs_run_device_noalloc(ccs_ctx *c, size_t n, const double *d_rnd,
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, block, 0));
   size_t grid = 0;
-  lane_shape(c, n, per_sm, grid, k.lane_width);
+  lane_shape(c, n, per_sm, G, grid, k.lane_width);
   CK(cudaEventRecord(c->ev[2], s));
   CK(cudaEventRecord(c->ev[5], s));
   fn<<<(unsigned)grid, block, 0, s>>>(k, kparams);
