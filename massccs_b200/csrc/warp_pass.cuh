@@ -335,6 +335,8 @@ template <typename T, int GAS, int NT> struct WarpShared {
   unsigned long long blk[8];
   unsigned long long idx;
   int kind, stop;
+  T ang[2];     // the usual steps' angle and whether it is left to angle3, alternating like red
+  int wide[2];
 };
 
 // The rounded square root of x without a branch (the usual call has one for
@@ -384,61 +386,87 @@ __device__ __forceinline__ void step_forces(const KParams &kp, const T (*red)[Wa
   absorb_forces<T, GAS>(kp, fs, L);
 }
 
-// Bounds that decide a step well inside the cutoffs without its exact reach
-// (a square root on the way to the forces): half the pair distance within
-// half a percent of its constrained value.
-template <typename T> struct StepBounds {
-  T offhi, hd2lo, hd2hi, rin2, rout2;
+// A ball in which every step is usual, however it is rounded: all sites
+// inside the reference grid, the probe inside the box and the ellipsoid and
+// within reach of the target, its candidates those at hand.  Each of these
+// is a bound on a function of the centre that changes by at most its
+// displacement, so one distance replaces all the tests of a step.
+template <typename T> struct Usual {
+  T c[3], rho2;        // the ball (rho2 < 0: none)
+  T hd2lo, hd2hi;      // the pair distance within half a percent of its constrained value
 };
+
+// The ball around c for the candidates at hand: a list (built around c, good
+// within LSKIN of it), or all atoms; everyone: all atoms whatever the distance.
+template <typename T, int GAS>
+__device__ __noinline__ T usual_radius2(const KParams *__restrict__ kpg, T cx, T cy, T cz, bool list, bool everyone) {
+  const KParams &kp = *kpg;
+  const KConst<T> &kc = kconst<T>(kp);
+  const T offm = GAS == GAS_ATOM ? T(0) : T(0.5) * T(sqrt(kc.d2)), offlo = offm * T(0.995), offhi = offm * T(1.005);
+  const T c[3] = {cx, cy, cz};
+  T e2 = T(0), f2 = T(0), u2 = T(0), rho = T(1e6);
+  const T half[3] = {kc.lx, kc.ly, kc.lz}, inv[3] = {kc.inv_a, kc.inv_b, kc.inv_c};
+  for (int k = 0; k < 3; k++) {
+    const T lo = kc.bb_lo[k] - c[k], hi = c[k] - kc.bb_hi[k];
+    const T e = fmax(fmax(lo, hi), T(0)), f = fmax(-lo, -hi);
+    e2 += e * e;
+    f2 += f * f;
+    u2 += c[k] * inv[k] * c[k] * inv[k];
+    rho = fmin(rho, fmin(kp.ref_check ? kc.ref_lim[k] - offhi : T(1e6), half[k]) - fabs(c[k]));
+  }
+  rho = fmin(rho, (T(1) - sqrt(u2)) / fmax(fmax(inv[0], inv[1]), inv[2]));
+  if (!kp.allpairs) {
+    const T rin = kc.reach + offlo, rout = kc.reach + offhi + T(0.01);
+    rho = fmin(rho, rin - sqrt(e2));
+    if (list) rho = fmin(rho, sqrt(f2) - rout);
+    else if (!everyone) rho = fmin(rho, rin - sqrt(f2));
+  }
+  rho -= T(2e-3);  // far more than any rounding here or there
+  if (!(rho > T(0))) return T(-1);
+  return list && rho >= T(LSKIN) ? T(LSKIN) * T(LSKIN) : rho * rho;
+}
+
 enum : int { F_OTHER = 0, F_TEST = 1, F_WIDE = 2 };
 
-// Usual steps, one after another: the probe inside the reach and the
-// reference grid, its candidates known (mode), no end of the try.  Few
-// branches, so that what is not on the way to the forces (the angle, the
-// tests) fills the latencies of what is.  One copy of the integrator for all
-// roles: every warp of the CTA computes the same bits and takes the same
-// turns.  Returns F_OTHER: a step whose move is done and which is not usual;
-// F_TEST: after a step, an exit test or the periodic check is due; F_WIDE:
-// the same with the step's angle still to do.
+// Usual steps, one after another: the probe in the ball, its candidates
+// known (mode), no end of the try.  Few branches, so that little stands
+// between the forces and the next positions.  One copy of the integrator for
+// all roles: every warp of the CTA computes the same bits and takes the same
+// turns; only the step's angle, which nothing waits for, is one warp's (the
+// role with the least to sum) and reaches the others with the forces.
+// Returns F_OTHER: a step whose move is done and which is not usual; F_TEST:
+// after a step, an exit test or the periodic check is due; F_WIDE: the same
+// with the step's angle still to do.
 template <typename T, int GAS, bool HASQ, int NT>
-__device__ __forceinline__ int usual_steps(int role, const KParams &kp, LaneState<T> &L, T inv_dt,
-                                           const StepBounds<T> &sb, int mode, bool small, const Cand &cd,
-                                           const Atom<T> (&sa)[2], const T (&list_c)[3], int vt, int lane, int v,
+__device__ __forceinline__ int usual_steps(int role, const KParams &kp, LaneState<T> &L, T inv_dt, const Usual<T> &us,
+                                           int mode, const Cand &cd, const Atom<T> (&sa)[2], int vt, int lane, int v,
                                            WarpShared<T, GAS, NT> &sm, int &red, unsigned &it) {
   constexpr int NS = GasShape<GAS>::NS;
-  const KConst<T> &kc = kconst<T>(kp);
-  const bool all = !cd.masked;
+  constexpr int ANGLE_ROLE = GAS == GAS_N2 && HASQ ? 2 : 0;
   for (;;) {
     first_half_move<T, GAS>(kp, L, inv_dt);
     const T c[3] = {centre<T, GAS>(L, 0), centre<T, GAS>(L, 1), centre<T, GAS>(L, 2)};
-    const T ex = fmax(fmax(kc.bb_lo[0] - c[0], c[0] - kc.bb_hi[0]), T(0));
-    const T ey = fmax(fmax(kc.bb_lo[1] - c[1], c[1] - kc.bb_hi[1]), T(0));
-    const T ez = fmax(fmax(kc.bb_lo[2] - c[2], c[2] - kc.bb_hi[2]), T(0));
-    const T fx = fmax(c[0] - kc.bb_lo[0], kc.bb_hi[0] - c[0]);
-    const T fy = fmax(c[1] - kc.bb_lo[1], kc.bb_hi[1] - c[1]);
-    const T fz = fmax(c[2] - kc.bb_lo[2], kc.bb_hi[2] - c[2]);
-    const T e2 = ex * ex + ey * ey + ez * ez, f2 = fx * fx + fy * fy + fz * fz;
-    const T dcx = c[0] - list_c[0], dcy = c[1] - list_c[1], dcz = c[2] - list_c[2];
+    const T dcx = c[0] - us.c[0], dcy = c[1] - us.c[1], dcz = c[2] - us.c[2];
     const T moved2 = Real<T>::fma(dcz, dcz, Real<T>::fma(dcx, dcx, Real<T>::mul(dcy, dcy)));
-    const T ux = c[0] * kc.inv_a, uy = c[1] * kc.inv_b, uz = c[2] * kc.inv_c;
-    const T ax = fabs(c[0]), ay = fabs(c[1]), az = fabs(c[2]);
-    bool ok = (e2 <= sb.rin2) & (ax + sb.offhi < kc.ref_lim[0]) & (ay + sb.offhi < kc.ref_lim[1]) &
-              (az + sb.offhi < kc.ref_lim[2]);
-    // strictly inside the box and the ellipsoid, with room for another rounding of outside_box's sum
-    ok &= (ax < kc.lx) & (ay < kc.ly) & (az < kc.lz) & (ux * ux + uy * uy + uz * uz < T(1) - T(1e-6));
-    ok &= small | (all ? f2 <= sb.rin2 : (f2 > sb.rout2) & (moved2 <= T(LSKIN) * T(LSKIN)));
+    bool ok = moved2 <= us.rho2;
     if constexpr (GAS != GAS_ATOM) {
       const T hd[3] = {L.r1[0] - L.r2[0], L.r1[1] - L.r2[1], L.r1[2] - L.r2[2]};
       const T hd2 = dot3(hd, hd);
-      ok &= (hd2 >= sb.hd2lo) & (hd2 <= sb.hd2hi);
+      ok &= (hd2 >= us.hd2lo) & (hd2 <= us.hd2hi);
     }
     if (!ok) return F_OTHER;
-    bool wide;
-    const T ang = small_angle(c, L.rold, wide);
     T p[NS][3];
     site_positions<T, GAS>(L, p);
     T f[3] = {T(0), T(0), T(0)}, E[3] = {T(0), T(0), T(0)}, G[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
     step_visits<T, GAS, HASQ, NT>(kp, role, p, (1u << NS) - 1u, mode, cd, sa, vt, f, E, G);
+    if (role == ANGLE_ROLE && v == 0) {
+      bool wide;
+      const T ang = small_angle(c, L.rold, wide);
+      if (lane == 0) {
+        sm.ang[red] = ang;
+        sm.wide[red] = wide;
+      }
+    }
     step_reduce<T, GAS, HASQ>(role, f, E, G, lane, sm.red[red][v]);
     __syncthreads();
     bool act[NS];
@@ -446,6 +474,8 @@ __device__ __forceinline__ int usual_steps(int role, const KParams &kp, LaneStat
     for (int k = 0; k < NS; k++) act[k] = true;
     T sum[Row<GAS>::N];
     step_forces<T, GAS, HASQ, NT>(kp, sm.red[red], act, L, sum);
+    const T ang = sm.ang[red];
+    const bool wide = sm.wide[red] != 0;
     red ^= 1;
     L.nvis += (uint32_t)cd.m;
     second_kick<T, GAS>(kp, L);
@@ -594,18 +624,14 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
       pack_end<GAS, NT>(K.natoms, tid, NTHREADS, sm_pos, sm_ab, sm_abc);
       __syncthreads();
     }
-    StepBounds<T> sb;
-    {
-      const T offm = GAS == GAS_ATOM ? T(0) : T(0.5) * T(sqrt(kc.d2)), offlo = offm * T(0.995);
-      sb.offhi = offm * T(1.005);
-      sb.hd2lo = T(4) * offlo * offlo;
-      sb.hd2hi = T(4) * sb.offhi * sb.offhi;
-      const T rin = K.allpairs ? T(INFINITY) : kc.reach + offlo, rout = kc.reach + sb.offhi + T(0.01);
-      sb.rin2 = rin * rin;
-      sb.rout2 = rout * rout;
-    }
+    Usual<T> us;
+    us.rho2 = T(-1);
+    us.c[0] = us.c[1] = us.c[2] = T(0);
+    us.hd2lo = kc.d2 * T(0.995 * 0.995);
+    us.hd2hi = kc.d2 * T(1.005 * 1.005);
     int mode = C_NONE;
-    bool usual = false;  // the last step was near: the next may be a usual one
+    bool usual = false;  // the next step may be a usual one
+    bool us_list = false;
     int list_n = -1;  // this trajectory's candidate list (none yet)
     T list_c[3] = {T(0), T(0), T(0)};
     T inv_dt = Real<T>::div(T(1), L.dt);
@@ -644,8 +670,7 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
         }
       }
       if (r == S_CONTINUE && usual && L.mode == M_STEP) {
-        const int u = usual_steps<T, GAS, HASQ, NT>(role, K, L, inv_dt, sb, mode, small, cd, sa, list_c, vt, lane, v, sm,
-                                                    red, it);
+        const int u = usual_steps<T, GAS, HASQ, NT>(role, K, L, inv_dt, us, mode, cd, sa, vt, lane, v, sm, red, it);
         if (u == F_WIDE) turn<T, GAS>(L);
         if (u != F_OTHER) {
           it--;  // the loop's own count
@@ -785,7 +810,16 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
           }
           red ^= 1;
           L.nvis += nvis;
-          usual = !chunked && cd.m > 0;
+          // the ball for the next steps: around the list's centre, or this position
+          usual = !chunked && cd.m > 0 && L.mode == M_STEP;
+          if (usual && (!cd.masked || list_c[0] != us.c[0] || list_c[1] != us.c[1] || list_c[2] != us.c[2] || !us_list)) {
+            us_list = cd.masked;
+            us.c[0] = us_list ? list_c[0] : cx;
+            us.c[1] = us_list ? list_c[1] : cy;
+            us.c[2] = us_list ? list_c[2] : cz;
+            us.rho2 = usual_radius2<T, GAS>(Kg, us.c[0], us.c[1], us.c[2], us_list, small);
+          }
+          usual = usual && us.rho2 > T(0);
         } else {
           T fs[NS][3];
 #pragma unroll
