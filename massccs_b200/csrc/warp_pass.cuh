@@ -488,6 +488,59 @@ __device__ __forceinline__ int usual_steps(int role, const KParams &kp, LaneStat
   }
 }
 
+// The ball around c in which the probe is out of reach of the whole target
+// and inside the box and the ellipsoid: a free flight.
+template <typename T, int GAS>
+__device__ __noinline__ T free_radius2(const KParams *__restrict__ kpg, T cx, T cy, T cz) {
+  const KParams &kp = *kpg;
+  const KConst<T> &kc = kconst<T>(kp);
+  if (kp.allpairs) return T(-1);
+  const T c[3] = {cx, cy, cz};
+  T e2 = T(0), u2 = T(0), rho = T(1e6);
+  const T half[3] = {kc.lx, kc.ly, kc.lz}, inv[3] = {kc.inv_a, kc.inv_b, kc.inv_c};
+  for (int k = 0; k < 3; k++) {
+    const T e = fmax(fmax(kc.bb_lo[k] - c[k], c[k] - kc.bb_hi[k]), T(0));
+    e2 += e * e;
+    u2 += c[k] * inv[k] * c[k] * inv[k];
+    rho = fmin(rho, half[k] - fabs(c[k]));
+  }
+  const T offhi = GAS == GAS_ATOM ? T(0) : T(0.5 * 1.005) * T(sqrt(kc.d2));
+  rho = fmin(rho, (T(1) - sqrt(u2)) / fmax(fmax(inv[0], inv[1]), inv[2]));
+  rho = fmin(rho, sqrt(e2) - (kc.reach + offhi + T(0.01))) - T(2e-3);
+  return rho > T(0) ? rho * rho : T(-1);
+}
+
+// Steps of a free flight: no force, no barrier.  Returns as usual_steps.
+template <typename T, int GAS>
+__device__ __forceinline__ int free_steps(const KParams &kp, LaneState<T> &L, T inv_dt, const Usual<T> &us, unsigned &it) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    L.f1[k] = T(0);
+    if constexpr (GAS != GAS_ATOM) L.f2[k] = T(0);
+  }
+  for (;;) {
+    first_half_move<T, GAS>(kp, L, inv_dt);
+    const T c[3] = {centre<T, GAS>(L, 0), centre<T, GAS>(L, 1), centre<T, GAS>(L, 2)};
+    const T dcx = c[0] - us.c[0], dcy = c[1] - us.c[1], dcz = c[2] - us.c[2];
+    bool ok = dcx * dcx + dcy * dcy + dcz * dcz <= us.rho2;
+    if constexpr (GAS != GAS_ATOM) {
+      const T hd[3] = {L.r1[0] - L.r2[0], L.r1[1] - L.r2[1], L.r1[2] - L.r2[2]};
+      const T hd2 = dot3(hd, hd);
+      ok &= (hd2 >= us.hd2lo) & (hd2 <= us.hd2hi);
+    }
+    if (!ok) return F_OTHER;
+    bool wide;
+    const T ang = small_angle(c, L.rold, wide);
+    second_kick<T, GAS>(kp, L);
+    it++;
+    if (wide) return F_WIDE;
+    L.dtheta += ang;
+#pragma unroll
+    for (int k = 0; k < 3; k++) L.rold[k] = c[k];
+    if ((L.dtheta > T(1.5 * PI_D)) | (L.stepcount >= kp.max_steps) | ((it & 255u) == 0)) return F_TEST;
+  }
+}
+
 // The sites' energies of a step that begins or ends a try, one warp per
 // virtual warp (the lead role's) in the order of the force sums, into
 // row[v][U..U + NS) of the reduction buffer.  Out of line: once or twice a try.
@@ -631,7 +684,7 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
     us.hd2hi = kc.d2 * T(1.005 * 1.005);
     int mode = C_NONE;
     bool usual = false;  // the next step may be a usual one
-    bool us_list = false;
+    bool us_list = false, us_free = false;
     int list_n = -1;  // this trajectory's candidate list (none yet)
     T list_c[3] = {T(0), T(0), T(0)};
     T inv_dt = Real<T>::div(T(1), L.dt);
@@ -670,7 +723,9 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
         }
       }
       if (r == S_CONTINUE && usual && L.mode == M_STEP) {
-        const int u = usual_steps<T, GAS, HASQ, NT>(role, K, L, inv_dt, us, mode, cd, sa, vt, lane, v, sm, red, it);
+        const int u = us_free ? free_steps<T, GAS>(K, L, inv_dt, us, it)
+                              : usual_steps<T, GAS, HASQ, NT>(role, K, L, inv_dt, us, mode, cd, sa, vt, lane, v, sm,
+                                                              red, it);
         if (u == F_WIDE) turn<T, GAS>(L);
         if (u != F_OTHER) {
           it--;  // the loop's own count
@@ -812,8 +867,9 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
           L.nvis += nvis;
           // the ball for the next steps: around the list's centre, or this position
           usual = !chunked && cd.m > 0 && L.mode == M_STEP;
-          if (usual && (!cd.masked || list_c[0] != us.c[0] || list_c[1] != us.c[1] || list_c[2] != us.c[2] || !us_list)) {
+          if (usual && (!cd.masked || us_free || list_c[0] != us.c[0] || list_c[1] != us.c[1] || list_c[2] != us.c[2] || !us_list)) {
             us_list = cd.masked;
+            us_free = false;
             us.c[0] = us_list ? list_c[0] : cx;
             us.c[1] = us_list ? list_c[1] : cy;
             us.c[2] = us_list ? list_c[2] : cz;
@@ -825,6 +881,12 @@ __global__ void __launch_bounds__(WarpShape<T, GAS, HASQ, NT>::THREADS, WarpShap
 #pragma unroll
           for (int s = 0; s < NS; s++) fs[s][0] = fs[s][1] = fs[s][2] = T(0);
           absorb_forces<T, GAS>(K, fs, L);
+          if (L.mode == M_STEP && !out) {
+            us_free = true;
+            us.c[0] = cx; us.c[1] = cy; us.c[2] = cz;
+            us.rho2 = free_radius2<T, GAS>(Kg, cx, cy, cz);
+            usual = us.rho2 > T(0);
+          }
         }
         if (L.mode == M_INIT) { L.Ei += L.U; L.mode = M_STEP; continue; }
         if (L.mode == M_RESTART) { L.mode = M_STEP; continue; }
