@@ -115,10 +115,10 @@ struct KParams {
   const struct KParams *ions;
   const unsigned long long *ion_start;
   int nions;
-  // speculative retries (see resume_kernel): records of trajectories that
-  // failed their second try in the warp pass, the outcome of each remaining
-  // try, and the phase of the warp-pass launch (0: parked trajectories,
-  // 1: the speculative tries); spec_rec == nullptr: no speculation
+  // speculative retries (see claim_item): records of trajectories whose
+  // tries run at once, the outcome of each, and the phase of the warp-pass
+  // launch (0: parked trajectories and the tries recorded meanwhile, 1: any
+  // tries left); spec_rec == nullptr: no speculation
   struct SpecRec *spec_rec;
   struct SpecOut *spec_out;
   unsigned long long *spec_count, *spec_next;
@@ -1155,12 +1155,13 @@ template <typename T> __device__ __forceinline__ bool outside_box(const KParams 
 //             its own).  Probes out of reach feel exactly zero force.  A lane
 //             whose trajectory passes `park_steps` integration steps saves the
 //             exact integrator state to HBM ("parks" it) and takes new work.
-//  warp pass  parked trajectories resume one per CTA (64 threads by
-//             default): the force phase of a step uses every thread and the
-//             integrator runs CTA-uniform, so the long trajectories (captured
-//             orbits with up to ~3e5 steps) advance at the lowest per-step
-//             latency instead of sharing a warp with 31 others; failed tries
-//             can run at once (speculative retries, see resume_kernel).
+//  warp pass  parked trajectories resume one per CTA (warp_pass.cuh): the
+//             sums of a step's force evaluation are spread over the CTA's
+//             warps and the integrator runs CTA-uniform, so the long
+//             trajectories (captured orbits with up to ~3e5 steps) advance
+//             at the lowest per-step latency instead of sharing a warp with
+//             31 others; failed tries run at once (speculative retries,
+//             below).
 //
 // Finished trajectories write status / 1-cos(chi) / steps / visits at their
 // own index.  Restarts rebuild the initial state from the trajectory's random
@@ -1174,12 +1175,12 @@ constexpr int BLOCK = 128;
 // spilled words cost: n2_complex 199 -> 161 ms, he_assembly 343 -> 294; 5
 // spill into the loops), else 3.  The learned field's warp pass: molecules
 // run 512 threads per SM (8 CTAs of 64 at <= 128 registers), atoms are left
-// unconstrained.
+// unconstrained; the plain one: WarpShape in warp_pass.cuh.
 #ifndef CCS_LANE_MIN_BLOCKS
 #define CCS_LANE_MIN_BLOCKS(T, G) (sizeof(T) == 4 && (G) == 32 ? 4 : 3)
 #endif
-#ifndef CCS_WARP_MIN_BLOCKS
-#define CCS_WARP_MIN_BLOCKS(T, nt, gas) ((gas) == GAS_ATOM || sizeof(T) == 8 ? 1 : 512 / (nt))
+#ifndef CCS_FIELD_MIN_BLOCKS
+#define CCS_FIELD_MIN_BLOCKS(nt, gas) ((gas) == GAS_ATOM ? 1 : 512 / (nt))
 #endif
 
 __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
@@ -1848,22 +1849,22 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS(T, G))
   if (threadIdx.x == 7 && blk[7]) atomicAdd(&kp.stats[6], blk[7]);
 }
 
-// Warp pass: parked trajectories resume one per CTA (all NT threads hold
-// the same state; the force phase is block-cooperative).
-//
 // Speculative retries.  A failed try restarts the trajectory from its
 // initial state with the step dt0/(k+1) (System.cpp:453-458); the tries of a
 // trajectory are therefore independent computations, and only the decision
 // which one counts is sequential.  Captured orbits fail try after try, each
-// longer than the last, and set the end of a run.  So once a warp-pass
-// trajectory has failed spec_from tries (phase 0), it is recorded and left;
-// a second launch (phase 1) runs each recorded trajectory's remaining tries
-// at once, one CTA each, from the same code; spec_resolve_kernel then walks
-// every record's tries in order with the reference's rules.  Every try runs
-// the same instructions as it would in sequence, so the results are those of
-// the sequential path.
-constexpr int RBLOCK = 64;  // default threads per trajectory in the warp pass
-
+// longer than the last, and set the end of a run.  So once a trajectory has
+// failed spec_from tries (the first by default; in either pass) and the warp
+// pass is short of work, it is recorded: its CTA goes on with the try at
+// hand, and CTAs without a parked trajectory take the later ones from the
+// record.  A try beyond one that decides is skipped, or stops within 256
+// steps.  spec_resolve_kernel then walks every record's tries in order with
+// the reference's rules.  Every try runs the same instructions as it would in
+// sequence, so the results are those of the sequential path.  Measured
+// against records from the second failure on, the trajectory's own CTA
+// leaving it, and every try run to its end (warp pass, ms): he_protein_100k
+// 44 -> 16, n2_allpairs_10k 143 -> 100, n2_fp64_1k 128 -> 62.
+constexpr int RBLOCK = 64;  // default (virtual) threads per trajectory in the warp pass
 
 // Thread 0's claim of the CTA's next item: a parked trajectory (kind 0), else
 // a speculative try (kind 1); ~0: none is left.
@@ -1979,13 +1980,16 @@ __device__ __forceinline__ unsigned long long record_spec(const KParams &kp, uns
   return slot;
 }
 
-// SURR: steps whose sites all lie outside the learned field's exact zone are
-// evaluated by the field, one warp per site (field_site_warp).
-template <typename T, int GAS, bool HASQ, int NT, bool BATCH, bool SURR = false>
-__global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_kernel(KParams kp, const KParams *__restrict__ kpg) {
+// The warp pass with the learned field (the plain one is warp_pass.cuh's):
+// one parked trajectory per CTA of NT threads, the force phase
+// block-cooperative; steps whose sites all lie outside the field's exact zone
+// are evaluated by the field, one warp per site (field_site_warp).
+template <int GAS, bool HASQ, int NT>
+__global__ void __launch_bounds__(NT, CCS_FIELD_MIN_BLOCKS(NT, GAS)) resume_field_kernel(KParams kp, const KParams *__restrict__ kpg) {
+  using T = float;
+  constexpr bool BATCH = false;
   using S = Sites<GAS>;
   constexpr int NS = S::NS;
-  static_assert(!SURR || (sizeof(T) == 4 && !BATCH), "the learned field runs in FP32 single-ion launches");
   __shared__ float sm_site[NS][4 * FL_SITE_FIELDS];
   extern __shared__ int sm_list[];  // kp.lcap entries (+ LCAP with the field; dynamic shared memory)
   __shared__ int sm_wsum[NT / 32];
@@ -2087,15 +2091,12 @@ __global__ void __launch_bounds__(NT, CCS_WARP_MIN_BLOCKS(T, NT, GAS)) resume_ke
           bool act[NS];
 #pragma unroll
           for (int s = 0; s < NS; s++) act[s] = (actbits >> s) & 1u;
-          bool surr = false;  // block-uniform: every thread holds the same state
-          if constexpr (SURR) {
-            surr = true;
+          bool surr = true;  // block-uniform: every thread holds the same state
 #pragma unroll
-            for (int s = 0; s < NS; s++)
-              if (act[s]) surr &= !field_exact(kp.field, (float)p[s][0], (float)p[s][1], (float)p[s][2]);
-          }
+          for (int s = 0; s < NS; s++)
+            if (act[s]) surr &= !field_exact(kp.field, (float)p[s][0], (float)p[s][1], (float)p[s][2]);
           if (surr) {
-            if constexpr (SURR) {
+            {
               // the switched exact sums over the atoms within r_out ...
               T raw[RedShape<GAS>::NV];
               T none;

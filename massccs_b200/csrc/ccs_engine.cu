@@ -116,11 +116,11 @@ KernelFn pick_traj(const ccs_ctx *c, int G) {
   return c->p.precision == CCS_PREC_FP64 ? pick_lane_t<double>(gas, hasq, G, false)
                                          : pick_lane_t<float>(gas, hasq, G, false);
 }
-// threads per trajectory in the warp pass
-// Threads per warp-pass trajectory: the configured value, else 32 for
-// molecules on targets whose candidate lists fit the smallest list (one warp
-// per trajectory, no cross-warp reduction: measured 1.90 against 1.98 s per
-// 3e5 trajectories on the 1231-atom N2 globule), else RBLOCK (64).
+// Virtual threads per warp-pass trajectory, i.e. how many partial sums the
+// candidates are dealt to (the order of the sums, and so the results' last
+// bits, depend on it): the configured value, else 32 for molecules on targets
+// whose candidate lists fit the smallest list, else RBLOCK (64).  The CTA has
+// a warp per role for each 32 of them.
 int resume_threads(const ccs_ctx *c) {
   const int b = c->p.resume_block;
   if (b == 32 || b == 64 || b == 128) return b;

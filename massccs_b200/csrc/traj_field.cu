@@ -18,9 +18,9 @@ template <int GAS, bool HASQ> ccs_internal::KernelFn traj_g(int G) {
   }
 }
 template <int GAS, bool HASQ> ccs_internal::KernelFn resume_nt(int nt) {
-  return nt == 32 ? resume_kernel<float, GAS, HASQ, 32, false, true>
-                  : nt == 128 ? resume_kernel<float, GAS, HASQ, 128, false, true>
-                              : resume_kernel<float, GAS, HASQ, 64, false, true>;
+  return nt == 32 ? resume_field_kernel<GAS, HASQ, 32>
+                  : nt == 128 ? resume_field_kernel<GAS, HASQ, 128>
+                              : resume_field_kernel<GAS, HASQ, 64>;
 }
 }  // namespace
 

@@ -8,8 +8,22 @@
 // force, the dipole's field, the field's gradient); each group of sums is a
 // role, and each role is a warp that walks the whole candidate list.  A sum's
 // order (which candidates a lane adds, and when) is that of one warp doing
-// all of them, so the split changes no result.  Measured on the 1231-atom N2
-// globule (about 1100 candidates a step): see the figures at warp_pass_kernel.
+// all of them (NT "virtual threads": thread t adds candidates t, t + NT, ...),
+// so the split changes no result.
+//
+// What bounds it: alone, the latency of a step (an instruction every 3.2
+// cycles and warp); with the SM full, instruction fetch and issue (0.59 a
+// cycle).  One step of one trajectory alone on the GPU, one warp (N2, CO2: 32
+// threads; else 64) doing all sums against this pass, us:
+//   He, 60 atoms 0.48 -> 0.26; He, 1231 atoms 1.08 -> 0.81; Ar, 777 atoms,
+//   LJ 0.78 -> 0.54; N2, 1231 atoms, +4 e 6.7 -> 1.5; CO2, 1001 atoms 6.7 ->
+//   1.3; N2, 20,000 atoms 6.7 -> 2.1; N2 in FP64 5.5 -> 2.2; N2 without
+//   cutoffs, 333 atoms 3.8 -> 1.3; He, shell of 5e5 atoms 5.4 -> 3.4.
+// Tried and left out: one integrating warp per CTA with the others waiting for
+// positions (N2 1.62 -> 1.76 us: its two hand-overs cost more than the copies
+// of the integrator), two candidates per instruction in packed FP32 (no gain:
+// the step is not short of multiply-adds), 2 or 8 candidates side by side
+// (2: 10 % slower on lists of thousands), 5 CTAs an SM (the registers spill).
 #pragma once
 
 #include "ccs_device.cuh"
