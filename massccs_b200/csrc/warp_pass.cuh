@@ -576,14 +576,17 @@ __device__ __noinline__ void warp_energy(const KParams *__restrict__ kpg, const 
   if (lead) reduce_group_row<T, 32, GAS, Row<GAS>::U, Row<GAS>::N>(acc, lane, 0xffffffffu, row);
 }
 
-// CTAs per SM that the register allocation allows: FP32 512 threads (128
-// registers), FP64 unconstrained.
-#ifndef CCS_WARP_THREADS_PER_SM
-#define CCS_WARP_THREADS_PER_SM 512
-#endif
+// CTAs per SM that the register allocation must allow, FP32: CTAs of up to
+// 128 threads share an SM by threes (168 registers: four candidates side by
+// side and the integrator's state fit), larger ones by twos (128).  Measured
+// against 512 threads an SM throughout: one lone step of N2 1.52 -> 1.33 us,
+// CO2 1.33 -> 1.19, He globule 0.81 -> 0.74; warp pass of n2_protein_3k 41 ->
+// 35 ms, co2_protein_9k 93 -> 82, n2_protein_150k (queue full for a third of
+// it) 360 -> 363; one CTA of 256 threads an SM takes n2_complex_20k from 260
+// to 300.  FP64 is unconstrained.
 template <typename T, int GAS, bool HASQ, int NT> struct WarpShape {
   static constexpr int THREADS = NT * Roles<GAS, HASQ>::N;
-  static constexpr int MINB = sizeof(T) == 8 ? 1 : (CCS_WARP_THREADS_PER_SM / THREADS > 0 ? CCS_WARP_THREADS_PER_SM / THREADS : 1);
+  static constexpr int MINB = sizeof(T) == 8 ? 1 : THREADS <= 128 ? 384 / THREADS : THREADS <= 256 ? 2 : 1;
 };
 
 // The warp pass.  See the speculative retries in ccs_device.cuh for the hand-
