@@ -255,6 +255,10 @@ int setup_spec(ccs_ctx *c, KParams &k, size_t cap, cudaStream_t s) {
   return CCS_OK;
 }
 
+// The most dynamic shared memory that any warp-pass launch asks for.
+constexpr int WP_SMEM_MAX = 60 * 1024;
+static_assert((LCAP_MAX + LCAP) * sizeof(int) <= WP_SMEM_MAX, "the learned field's two lists do not fit");
+
 // Grid and shared memory of a warp-pass kernel, with the sizes that the
 // kernel reads (k.lcap set): the candidate list, its packed copy where that
 // leaves room for four CTAs on an SM (FP32, lists of up to about 2000
@@ -268,13 +272,16 @@ int warp_shape(ccs_ctx *c, const WarpKernel &wk, KParams &k, size_t most_atoms, 
     dyn = ((size_t)k.wp_cap * sizeof(int) + 15) / 16 * 16;
     const int places = (k.wp_cap + WP_BLOCK - 1) / WP_BLOCK * WP_BLOCK;  // whole blocks
     const size_t packed = (size_t)places * (sizeof(float4) + (c->p.gas == CCS_GAS_CO2 ? 2 : 1) * sizeof(float2));
-    if (c->p.precision != CCS_PREC_FP64 && dyn + packed <= 60 * 1024) {
+    if (c->p.precision != CCS_PREC_FP64 && dyn + packed <= WP_SMEM_MAX) {
       k.wp_pack = places;
       dyn += packed;
     }
   }
+  // The attribute belongs to the kernel on this device, not to the context, and
+  // other threads' contexts launch the same kernel: always the one largest
+  // value, so that no run lowers what another is about to launch with.
   if (dyn > 32 * 1024)
-    CK(cudaFuncSetAttribute((const void *)wk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    CK(cudaFuncSetAttribute((const void *)wk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM_MAX));
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)wk.fn, wk.threads, dyn));
   grid = (size_t)std::max(per_sm, 1) * c->sm_count;
