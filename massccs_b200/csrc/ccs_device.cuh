@@ -203,7 +203,7 @@ __device__ __forceinline__ SpecRec load_spec_rec(const SpecRec *p) {
   R.nvis = __ldcg(&p->nvis);
   R.tries = __ldcg(&p->tries);
   R.maxTries = __ldcg(&p->maxTries);
-  R.stop = *(const volatile int *)&p->stop;
+  R.stop = 9;  // it changes while tries run: one thread reads it for the CTA
   R.ended = R.energy = 0;
   R.ready = 1;
   return R;
@@ -1864,6 +1864,9 @@ __global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS(T, G))
 // against records from the second failure on, the trajectory's own CTA
 // leaving it, and every try run to its end (warp pass, ms): he_protein_100k
 // 44 -> 16, n2_allpairs_10k 143 -> 100, n2_fp64_1k 128 -> 62.
+// With the learned field (20,000 atoms, 10,000 trajectories, s), every try run
+// to its end against needless ones skipped or stopped: N2 6.1 -> 2.7, CO2
+// 5.3 -> 3.4; tries in sequence 2.5 and 9.5.
 constexpr int RBLOCK = 64;  // default (virtual) threads per trajectory in the warp pass
 
 // Thread 0's claim of the CTA's next item: a parked trajectory (kind 0), else
@@ -2023,7 +2026,7 @@ __global__ void __launch_bounds__(NT, CCS_FIELD_MIN_BLOCKS(NT, GAS)) resume_fiel
   // launch runs whatever is left (records beyond this, or after a timeout).
   // The wait polls with a sleep and ends at the watchdog's deadline.
   bool park_done = spec_launch;
-  __shared__ int sm_kind;
+  __shared__ int sm_kind, sm_stop;
   for (;;) {
     if (tid == 0) {
       int kind;
@@ -2039,9 +2042,13 @@ __global__ void __launch_bounds__(NT, CCS_FIELD_MIN_BLOCKS(NT, GAS)) resume_fiel
     unsigned long long rec = 0;
     if (spec) {  // try k of record rec, from the trajectory's initial state
       rec = idx / SPEC_ITEMS;
+      if (tid == 0) sm_stop = *(volatile int *)&kp.spec_rec[rec].stop;
+      __syncthreads();
+      const int stop = sm_stop;
+      __syncthreads();
       const SpecRec R = load_spec_rec(kp.spec_rec + rec);
       const int k = R.tries + 1 + (int)(idx % SPEC_ITEMS);
-      if (k > 8) continue;  // beyond the reference's last try (block-uniform)
+      if (k > 8 || k > stop) continue;  // beyond the last try, or decided before it (block-uniform)
       L.j = R.j;
       L.ion = R.ion;
       load_init<T, GAS>(L, lane_setup<T, GAS>(ion_params_ptr<BATCH>(kp, kpg, L.ion), L.j));
@@ -2067,11 +2074,16 @@ __global__ void __launch_bounds__(NT, CCS_FIELD_MIN_BLOCKS(NT, GAS)) resume_fiel
     for (unsigned it = 1;; it++) {
       int r = S_CONTINUE;
       double omc = 0.0;
-      if ((it & 1023u) == 0) {
-        if (tid == 0) sm_idx = (global_ns() > deadline || *(volatile int *)kp.error) ? 1ull : 0ull;
+      if ((it & 255u) == 0) {
+        if (tid == 0) {
+          sm_stop = (global_ns() > deadline || *(volatile int *)kp.error)                   ? 1
+                    : spec && L.tries > *(volatile int *)&kp.spec_rec[rec].stop ? 2
+                                                                                : 0;
+        }
         __syncthreads();
-        const bool e = sm_idx != 0;
+        const int e = sm_stop;
         __syncthreads();
+        if (e == 2) break;  // the trajectory is decided by an earlier try
         if (e) {
           if (tid == 0) atomicExch(kp.error, 1);
           r = S_CAPPED;
