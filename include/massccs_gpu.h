@@ -101,8 +101,10 @@ typedef struct {
   int32_t resume_block;     /* partial sums per force evaluation in the warp pass: 32, 64 or 128
                                (results at rounding level depend on it); 0 = 32 for N2/CO2 in FP32
                                on targets whose candidate lists fit 2048 entries, else 64 */
-  int32_t spec_tries;       /* failed tries after which a warp-pass trajectory runs its remaining
-                               tries at once (2..8); 0 = default, < 0 = never */
+  int32_t spec_tries;       /* failed tries, in either pass, after which a trajectory in the warp
+                               pass runs its remaining tries at once when that pass is short of
+                               work (1..8; with the learned field, from a try that fails in the
+                               warp pass on); 0 = 1, < 0 = never */
 } ccs_params;
 
 /* Per-run statistics. */

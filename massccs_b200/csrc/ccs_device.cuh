@@ -1176,12 +1176,8 @@ constexpr int BLOCK = 128;
 // spill into the loops), else 3.  The learned field's warp pass: molecules
 // run 512 threads per SM (8 CTAs of 64 at <= 128 registers), atoms are left
 // unconstrained; the plain one: WarpShape in warp_pass.cuh.
-#ifndef CCS_LANE_MIN_BLOCKS
-#define CCS_LANE_MIN_BLOCKS(T, G) (sizeof(T) == 4 && (G) == 32 ? 4 : 3)
-#endif
-#ifndef CCS_FIELD_MIN_BLOCKS
-#define CCS_FIELD_MIN_BLOCKS(nt, gas) ((gas) == GAS_ATOM ? 1 : 512 / (nt))
-#endif
+template <typename T, int G> constexpr int lane_min_blocks() { return sizeof(T) == 4 && G == 32 ? 4 : 3; }
+constexpr int field_min_blocks(int nt, int gas) { return gas == GAS_ATOM ? 1 : 512 / nt; }
 
 __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
   for (int k = 0; k < n; k++) m &= m - 1u;
@@ -1510,7 +1506,7 @@ __device__ __forceinline__ const KParams *ion_params_ptr(const KParams &kp, cons
 // MLP tile spans the CTA's 128 lanes; probes in the exact zone take the
 // exact path below as before.
 template <typename T, int G, int GAS, bool HASQ, bool BATCH, bool SURR = false>
-__global__ void __launch_bounds__(BLOCK, SURR ? 2 : CCS_LANE_MIN_BLOCKS(T, G))
+__global__ void __launch_bounds__(BLOCK, SURR ? 2 : lane_min_blocks<T, G>())
     traj_kernel(KParams kp, const KParams *__restrict__ kpg) {
   using S = Sites<GAS>;
   constexpr int NS = S::NS;
@@ -1988,7 +1984,7 @@ __device__ __forceinline__ unsigned long long record_spec(const KParams &kp, uns
 // block-cooperative; steps whose sites all lie outside the field's exact zone
 // are evaluated by the field, one warp per site (field_site_warp).
 template <int GAS, bool HASQ, int NT>
-__global__ void __launch_bounds__(NT, CCS_FIELD_MIN_BLOCKS(NT, GAS)) resume_field_kernel(KParams kp, const KParams *__restrict__ kpg) {
+__global__ void __launch_bounds__(NT, field_min_blocks(NT, GAS)) resume_field_kernel(KParams kp, const KParams *__restrict__ kpg) {
   using T = float;
   constexpr bool BATCH = false;
   using S = Sites<GAS>;

@@ -260,10 +260,15 @@ constexpr int WP_SMEM_MAX = 60 * 1024;
 static_assert((LCAP_MAX + LCAP) * sizeof(int) <= WP_SMEM_MAX, "the learned field's two lists do not fit");
 
 // Grid and shared memory of a warp-pass kernel, with the sizes that the
-// kernel reads (k.lcap set): the candidate list, its packed copy where that
-// leaves room for four CTAs on an SM (FP32, lists of up to about 2000
-// candidates: a step then reads 24 B in list order instead of an index and a
-// gather), and with the learned field the near-part list.
+// kernel reads (k.lcap set): the candidate list, its packed copy where both
+// fit in WP_SMEM_MAX, three CTAs on an SM, which is what the registers of a
+// 128-thread CTA allow too (FP32, lists of up to 2048 candidates, CO2 1536: a
+// step then reads 24 B, CO2 32, in list order instead of an index and a
+// gather), and with the learned field the near-part list.  64-thread CTAs
+// (no charges) could sit by sixes without the copy, but three with it are
+// faster: warp pass, indices only -> packed, Ar on 2000 atoms (30,000
+// trajectories) 28.1 -> 27.1 ms, N2 on 2500 (20,000) 24.0 -> 21.8 and on 5000
+// (60,000) 18.9 -> 16.8.
 int warp_shape(ccs_ctx *c, const WarpKernel &wk, KParams &k, size_t most_atoms, size_t &grid, size_t &dyn) {
   k.wp_cap = (int)((std::min<size_t>(k.lcap, most_atoms) + 3) / 4 * 4);
   k.wp_pack = 0;
@@ -477,7 +482,12 @@ int read_stats(ccs_ctx *c, ccs_stats *st, size_t n) {
 }
 
 // Autotuner: times each lanes-per-trajectory choice on a slice of the run and
-// keeps the fastest (trajectories are independent, so a slice is a fair sample).
+// keeps the fastest.  The slice is spread over the warps like a run of its own
+// size, so a large run's warps are fuller than the slice's; that has not moved
+// the choice: 32 lanes are fastest in slices and in whole runs alike (60 atoms,
+// He, 3e5 trajectories: lane pass 6.1 ms, next 10.8 with 16 lanes; 1231 atoms,
+// He, 1e5: 34 and 59; N2, 1.5e5: 202 and 325; 777 atoms, Ar, 12,345: 11 and 15;
+// 333 atoms, N2 without cutoffs, 1e4: 41 and 42).
 int autotune(ccs_ctx *c, size_t n, size_t stride, int block) {
   if (c->p.lanes_per_traj > 0) { c->tuned_G = c->p.lanes_per_traj; c->tuned_block = block; return CCS_OK; }
   if (c->tuned_G) return CCS_OK;

@@ -13,12 +13,13 @@
 //
 // What bounds it: alone, the latency of a step (an instruction every 3.2
 // cycles and warp); with the SM full, instruction fetch and issue (0.59 a
-// cycle).  One step of one trajectory alone on the GPU, one warp (N2, CO2: 32
-// threads; else 64) doing all sums against this pass, us:
-//   He, 60 atoms 0.48 -> 0.26; He, 1231 atoms 1.08 -> 0.81; Ar, 777 atoms,
-//   LJ 0.78 -> 0.54; N2, 1231 atoms, +4 e 6.7 -> 1.5; CO2, 1001 atoms 6.7 ->
-//   1.3; N2, 20,000 atoms 6.7 -> 2.1; N2 in FP64 5.5 -> 2.2; N2 without
-//   cutoffs, 333 atoms 3.8 -> 1.3; He, shell of 5e5 atoms 5.4 -> 3.4.
+// cycle).  One step of one trajectory alone on the GPU, us: 32 (N2, CO2) or 64
+// threads doing all sums, the energies at every step among them -> this pass:
+//   He, 60 atoms 0.48 -> 0.25; He, 1231 atoms 1.08 -> 0.74; Ar, 777 atoms,
+//   LJ 0.78 -> 0.53; N2, 1231 atoms, +4 e 6.7 -> 1.34; CO2, 1001 atoms 6.7 ->
+//   1.18; N2, 20,000 atoms 6.7 -> 2.14; N2 in FP64 5.5 -> 2.2; N2 without
+//   cutoffs, 333 atoms 3.8 -> 1.26; He, shell of 5e5 atoms 5.3 -> 2.8.
+// (Without the energies at every step the former took 3.3 us for the N2 one.)
 // Tried and left out: one integrating warp per CTA with the others waiting for
 // positions (N2 1.62 -> 1.76 us: its two hand-overs cost more than the copies
 // of the integrator), two candidates per instruction in packed FP32 (no gain:
@@ -76,6 +77,7 @@ __device__ __forceinline__ void visit_role(const KParams &kp, const T (&p)[3], T
     const bool in_c = r2 < kc.rc2;
     const T ir3 = Real<T>::mul(ir, ir2);
     const T ir3s = Real<T>::add(ir3, -kc.rc3inv);
+    // (an ion without Coulomb forces has no charges in its table: ccs_set_target)
     if constexpr (RO::force(R) && site_coul<GAS>(s)) {
       T ir3c = Real<T>::fma(ir, ir2, -kc.rc3inv);
       if constexpr (s == GasShape<GAS>::DIP) ir3c = dipf ? ir3c : ir3s;
